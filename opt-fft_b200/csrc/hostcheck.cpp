@@ -10,11 +10,13 @@
 #include <string.h>
 
 #include <algorithm>
+#include <array>
 #include <vector>
 
 #include "staged.cuh"
 #include "mgpu.cuh"
 #include "splitline.cuh"
+#include "recycle.cuh"
 #include "twopass.cuh"
 #include "volume.cuh"
 
@@ -398,6 +400,51 @@ static void emulate_twopass_staged(const void *vin, void *vout, long long nvol)
     }
 }
 
+// The RECYCLE kernels (recycle_kernels.cu k_recycle; recycle.cuh) on a grid of
+// 3 CTAs: a chunk's rows of the following planes overwrite the ring as soon as
+// its x lines are in registers, before the remaining chunks are read.
+template <int N0, int N1, int N2, typename T, int S, int PITCH, int NP, int RC>
+static void emulate_recycle(const void *vin, void *vout, long long nvol)
+{
+    using RG = Recycle<N0, N1, N2, T, PITCH, NP, RC>;
+    using G = typename RG::G;
+    const T scale = S > 0 ? T(1) / T(G::V) : T(1);
+    const cx<T> *in = (const cx<T> *)vin;
+    cx<T> *out = (cx<T> *)vout;
+    std::vector<cx<T>> sm((size_t)NP * N1 * PITCH, cx<T>{T(12345.0), T(-6789.0)});
+    for (long long cta = 0; cta < 3; ++cta) {
+        const long long mine = nvol > cta ? (nvol - cta + 2) / 3 : 0;
+        auto issue = [&](long long q, int c, int yy) {
+            const long long k = q / N0;
+            if (k >= mine) return;
+            const int x = (int)(q % N0), s = (int)(q % NP), y = c * RC + yy;
+            const cx<T> *src = in + (cta + k * 3) * G::V + (x * N1 + y) * N2;
+            for (int z = 0; z < N2; ++z) sm[G::off(s * N1 + y, z)] = src[z];
+        };
+        for (int c = 0; c < RG::C; ++c)
+            for (int i = 0; i < NP * RG::rows(c); ++i) issue(i / RG::rows(c), c, i % RG::rows(c));
+        int base = 0;
+        for (long long k = 0; k < mine; ++k) {
+            for (int t = 0; t < G::ROWS; ++t) {
+                int x, y, c;
+                RG::z_row(t, &x, &y, &c);
+                pass_z<G, S, 0>(sm.data(), RG::slot(base, x) * N1 + y);
+            }
+            for (int l = 0; l < N0 * N2; ++l) pass_y<G, S, 0>(sm.data(), RG::slot(base, l / N2) * N2 + l % N2);
+            cx<T> *gout = out + (cta + k * 3) * G::V;
+            for (int c = 0; c < RG::C; ++c) {
+                const int lines = RG::rows(c) * N2;
+                std::vector<std::array<cx<T>, N0>> v(lines);
+                for (int l = 0; l < lines; ++l) RG::x_load(sm.data(), base, c, l, *(cx<T>(*)[N0])v[l].data());
+                for (int i = 0; i < N0 * RG::rows(c); ++i)
+                    issue(k * N0 + NP + i / RG::rows(c), c, i % RG::rows(c));
+                for (int l = 0; l < lines; ++l)
+                    RG::template x_store<S, 0>(gout, c, l, *(cx<T>(*)[N0])v[l].data(), scale);
+            }
+            base = RG::slot(base, N0 % NP);
+        }
+    }
+}
 
 typedef void (*emu_fn)(const void *, void *, long long);
 
@@ -415,6 +462,9 @@ typedef void (*emu_fn)(const void *, void *, long long);
 #define EMU_TPST(LINE, N, T)                                                                  \
     {N, N, N, sizeof(T) == 8 ? 0 : 1, -1, 701, 1, &emulate_twopass_staged<LINE, -1, T>},         \
     {N, N, N, sizeof(T) == 8 ? 0 : 1, +1, 701, 1, &emulate_twopass_staged<LINE, +1, T>}
+#define EMU_REC(N0, N1, N2, T, PITCH, NP, RC)                                                 \
+    {N0, N1, N2, sizeof(T) == 8 ? 0 : 1, -1, 900 + NP, RC, &emulate_recycle<N0, N1, N2, T, -1, PITCH, NP, RC>}, \
+    {N0, N1, N2, sizeof(T) == 8 ? 0 : 1, +1, 900 + NP, RC, &emulate_recycle<N0, N1, N2, T, +1, PITCH, NP, RC>}
 #define EMU_TP(N0, N1, N2, T, G)                                                              \
     {N0, N1, N2, sizeof(T) == 8 ? 0 : 1, -1, 300 + G, 1,                                    \
      &emulate_twopass<N0, N1, N2, T, -1, G>},                                                \
@@ -467,6 +517,9 @@ static const EmuEntry kEmu[] = {
     EMU_TPR(36, 36, 36, 3), EMU_TPR(36, 36, 36, 2), EMU_TPR(36, 36, 36, 4), EMU_TPRQ(36, 36, 36, 3),
     EMU_TPRQ(36, 36, 36, 2), EMU_TPRQ(6, 9, 5, 3), EMU_TPRQF(3), EMU_TPRQF(2), EMU_TPRQF(4), EMU_TPST(LineCT64, 64, double), EMU_TPST(LineCT64, 64, float), EMU_TPST(LinePFA45, 45, double),
     EMU_TPR(6, 9, 5, 3),
+    EMU_REC(16, 16, 32, double, 33, 27, 8), EMU_REC(23, 23, 23, double, 23, 23, 12),
+    EMU_REC(23, 23, 23, double, 23, 27, 12), EMU_REC(24, 24, 24, double, 25, 24, 8),
+    EMU_REC(30, 30, 30, float, 30, 30, 10), EMU_REC(16, 16, 16, double, 17, 16, 8),
     EMU_TPL(36, 2, 2), EMU_TPL(36, 2, 4), EMU_TPL(36, 1, 4), EMU_TPL(36, 3, 4),
     // the group sizes the VOLUME kernels of these extents use
     EMU(1, 1, 1, double, 0, 64),  EMU(3, 3, 3, double, 0, 32),   EMU(4, 4, 4, double, 0, 16),
@@ -708,6 +761,20 @@ extern "C" int hostcheck_tpass(int tl, int sign, void *data, long long vol_elems
 
 // Items whose dependency wait would not hold when taken in ticket order (the
 // TWOPASS deadlock-freedom argument); reset by reading.
+// LitTw<n> and the table's entries of length n, {cos, sin} each.
+extern "C" int hostcheck_literal_factors(int n, double *lit, double *tab)
+{
+    if (n != 19 && n != 23) return 1;
+    ensure_host_tables();
+    for (int e = 0; e < n; ++e) {
+        lit[2 * e] = n == 19 ? LitTw<19>::c(e) : LitTw<23>::c(e);
+        lit[2 * e + 1] = n == 19 ? LitTw<19>::s(e) : LitTw<23>::s(e);
+        tab[2 * e] = h_tw_d[tw_off(n) + e].x;
+        tab[2 * e + 1] = h_tw_d[tw_off(n) + e].y;
+    }
+    return 0;
+}
+
 extern "C" long long hostcheck_twopass_violations()
 {
     const long long v = g_twopass_violations;

@@ -46,6 +46,7 @@ const std::vector<KernelEntry> &registry()
     std::call_once(once, [] {
         register_stream_kernels(reg);
         register_stream_odd_kernels(reg);
+        register_recycle_kernels(reg);
         register_direct_kernels(reg);
         register_tc_kernels(reg);
         register_kernels(reg);

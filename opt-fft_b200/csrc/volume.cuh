@@ -49,9 +49,7 @@ FFT_HD void pass_z(cx<typename G::T> *sm, int r)
     cx<T> v[G::N2];
 #pragma unroll
     for (int j = 0; j < G::N2; ++j) v[j] = sm[G::off(r, j)];
-    dft<G::N2, S, T, ALG>(v);
-#pragma unroll
-    for (int j = 0; j < G::N2; ++j) sm[G::off(r, j)] = v[j];
+    dft_emit<G::N2, S, T, ALG>(v, [&](int j, cx<T> x) { sm[G::off(r, j)] = x; });
 }
 
 // Pass along z for row r read straight from HBM: rows are contiguous in the
@@ -66,9 +64,7 @@ FFT_HD void pass_z_from_global(cx<typename G::T> *sm, const cx<typename G::T> *g
     const cx<T> *p = gin + (long long)r * G::N2;
 #pragma unroll
     for (int j = 0; j < G::N2; ++j) v[j] = load_in(p + j);
-    dft<G::N2, S, T, ALG>(v);
-#pragma unroll
-    for (int j = 0; j < G::N2; ++j) sm[G::off(r, j)] = v[j];
+    dft_emit<G::N2, S, T, ALG>(v, [&](int j, cx<T> x) { sm[G::off(r, j)] = x; });
 }
 
 // Pass along y for line l = (vol*N0 + x)*N2 + z.
@@ -81,9 +77,7 @@ FFT_HD void pass_y(cx<typename G::T> *sm, int l)
     cx<T> v[G::N1];
 #pragma unroll
     for (int j = 0; j < G::N1; ++j) v[j] = sm[G::off(rb + j, z)];
-    dft<G::N1, S, T, ALG>(v);
-#pragma unroll
-    for (int j = 0; j < G::N1; ++j) sm[G::off(rb + j, z)] = v[j];
+    dft_emit<G::N1, S, T, ALG>(v, [&](int j, cx<T> x) { sm[G::off(rb + j, z)] = x; });
 }
 
 // Pass along x for line l = (vol*N1 + y)*N2 + z, read from shared memory and
@@ -172,15 +166,12 @@ FFT_HD void pass_x_out(const cx<typename G::T> *sm, int l, cx<typename G::T> *go
         cx<T> v[G::N0];
 #pragma unroll
         for (int j = 0; j < G::N0; ++j) v[j] = sm[G::off((vol * G::N0 + j) * G::N1 + y, z)];
-        dft<G::N0, S, T, ALG>(v);
         cx<T> *o = gout + (long long)vol * G::V + y * G::N2 + z;
-#pragma unroll
-        for (int j = 0; j < G::N0; ++j) {
-            cx<T> r = v[j];
+        dft_emit<G::N0, S, T, ALG>(v, [&](int j, cx<T> r) {
             if constexpr (S > 0) r = cscale(r, scale);
             if constexpr (KEEP) o[j * (G::N1 * G::N2)] = r;
             else store_out(o + j * (G::N1 * G::N2), r);
-        }
+        });
     }
 }
 
@@ -199,13 +190,10 @@ FFT_HD void pass_x(cx<typename G::T> *sm, int l, typename G::T scale)
     cx<T> v[G::N0];
 #pragma unroll
     for (int j = 0; j < G::N0; ++j) v[j] = sm[G::off((vol * G::N0 + j) * G::N1 + y, z)];
-    dft<G::N0, S, T, ALG>(v);
-#pragma unroll
-    for (int j = 0; j < G::N0; ++j) {
-        cx<T> r = v[j];
+    dft_emit<G::N0, S, T, ALG>(v, [&](int j, cx<T> r) {
         if constexpr (S > 0) r = cscale(r, scale);
         sm[G::off((vol * G::N0 + j) * G::N1 + y, z)] = r;
-    }
+    });
 }
 
 // Pass along x for line l into registers (scaled for the inverse), and the
