@@ -16,6 +16,7 @@
 #include "staged.cuh"
 #include "mgpu.cuh"
 #include "splitline.cuh"
+#include "longline.cuh"
 #include "recycle.cuh"
 #include "twopass.cuh"
 #include "volume.cuh"
@@ -446,6 +447,36 @@ static void emulate_recycle(const void *vin, void *vout, long long nvol)
     }
 }
 
+// The LONG kernels (long_kernels.cu k_long; longline.cuh): every task's sums of
+// a group of volumes before any output is put back.
+template <int N0, int N1, int N2, typename T, int S, int VPC, int KT>
+static void emulate_long(const void *vin, void *vout, long long nvol)
+{
+    using G = Geom<N0, N1, N2, T>;
+    using LL = LongLine<G, VPC, KT>;
+    const T scale = S > 0 ? T(1) / T(G::V) : T(1);
+    std::vector<cx<T>> sm((size_t)VPC * G::PV);
+    cx<double> tw[N0];
+    for (int e = 0; e < N0; ++e) {
+        const auto w = line_tw<N0, double>(e);
+        tw[e] = {w.x, w.y};
+    }
+    for (long long v0 = 0; v0 < nvol; v0 += VPC) {
+        const int nv = (int)std::min<long long>(VPC, nvol - v0);
+        const cx<T> *gin = (const cx<T> *)vin + v0 * G::V;
+        cx<T> *gout = (cx<T> *)vout + v0 * G::V;
+        for (int g = 0; g < nv * G::V; ++g) stage_in<G>(sm.data(), gin, g);
+        for (int r = 0; r < nv * G::ROWS; ++r) pass_z<G, S, 0>(sm.data(), r);
+        for (int l = 0; l < nv * N0 * N2; ++l) pass_y<G, S, 0>(sm.data(), l);
+        std::vector<typename LL::Acc> acc(LL::TASKS);
+        for (int t = 0; t < LL::TASKS; ++t)
+            if (t % LL::LINES < nv * N1 * N2) LL::sums(sm.data(), tw, t, acc[t]);
+        for (int t = 0; t < LL::TASKS; ++t)
+            if (t % LL::LINES < nv * N1 * N2) LL::template put<S>(sm.data(), t, acc[t], scale);
+        for (int g = 0; g < nv * G::V; ++g) gout[g] = sm[G::off(g / N2, g % N2)];
+    }
+}
+
 typedef void (*emu_fn)(const void *, void *, long long);
 
 #define EMU_TPR_(N0, N1, N2, G, A, XB)                                                       \
@@ -465,6 +496,9 @@ typedef void (*emu_fn)(const void *, void *, long long);
 #define EMU_REC(N0, N1, N2, T, PITCH, NP, RC)                                                 \
     {N0, N1, N2, sizeof(T) == 8 ? 0 : 1, -1, 900 + NP, RC, &emulate_recycle<N0, N1, N2, T, -1, PITCH, NP, RC>}, \
     {N0, N1, N2, sizeof(T) == 8 ? 0 : 1, +1, 900 + NP, RC, &emulate_recycle<N0, N1, N2, T, +1, PITCH, NP, RC>}
+#define EMU_LONG(N0, N1, N2, T, VPC, KT)                                                      \
+    {N0, N1, N2, sizeof(T) == 8 ? 0 : 1, -1, 2000 + KT, VPC, &emulate_long<N0, N1, N2, T, -1, VPC, KT>}, \
+    {N0, N1, N2, sizeof(T) == 8 ? 0 : 1, +1, 2000 + KT, VPC, &emulate_long<N0, N1, N2, T, +1, VPC, KT>}
 #define EMU_TP(N0, N1, N2, T, G)                                                              \
     {N0, N1, N2, sizeof(T) == 8 ? 0 : 1, -1, 300 + G, 1,                                    \
      &emulate_twopass<N0, N1, N2, T, -1, G>},                                                \
@@ -520,6 +554,8 @@ static const EmuEntry kEmu[] = {
     EMU_REC(16, 16, 32, double, 33, 27, 8), EMU_REC(23, 23, 23, double, 23, 23, 12),
     EMU_REC(23, 23, 23, double, 23, 27, 12), EMU_REC(24, 24, 24, double, 25, 24, 8),
     EMU_REC(30, 30, 30, float, 30, 30, 10), EMU_REC(16, 16, 16, double, 17, 16, 8),
+    EMU_LONG(97, 2, 1, double, 16, 6), EMU_LONG(83, 2, 1, double, 16, 6), EMU_LONG(47, 3, 2, double, 8, 8),
+    EMU_LONG(97, 2, 1, float, 16, 4), EMU_LONG(83, 2, 1, float, 16, 7), EMU_LONG(47, 3, 2, float, 8, 8),
     EMU_TPL(36, 2, 2), EMU_TPL(36, 2, 4), EMU_TPL(36, 1, 4), EMU_TPL(36, 3, 4),
     // the group sizes the VOLUME kernels of these extents use
     EMU(1, 1, 1, double, 0, 64),  EMU(3, 3, 3, double, 0, 32),   EMU(4, 4, 4, double, 0, 16),

@@ -60,6 +60,7 @@ void register_kernels(std::vector<KernelEntry> &out);          // volume_kernels
 void register_stream_kernels(std::vector<KernelEntry> &out);   // stream_kernels.cu
 void register_stream_odd_kernels(std::vector<KernelEntry> &out);  // stream_odd_kernels.cu
 void register_recycle_kernels(std::vector<KernelEntry> &out);     // recycle_kernels.cu
+void register_long_kernels(std::vector<KernelEntry> &out);        // long_kernels.cu
 void register_direct_kernels(std::vector<KernelEntry> &out);   // direct_kernels.cu
 void register_tc_kernels(std::vector<KernelEntry> &out);       // tc_kernels.cu
 int tc_tables_upload();                                         // split-BF16 DFT matrices

@@ -47,6 +47,7 @@ const std::vector<KernelEntry> &registry()
         register_stream_kernels(reg);
         register_stream_odd_kernels(reg);
         register_recycle_kernels(reg);
+        register_long_kernels(reg);
         register_direct_kernels(reg);
         register_tc_kernels(reg);
         register_kernels(reg);
