@@ -18,6 +18,7 @@
 #include "splitline.cuh"
 #include "longline.cuh"
 #include "recycle.cuh"
+#include "trip.cuh"
 #include "twopass.cuh"
 #include "volume.cuh"
 
@@ -477,6 +478,61 @@ static void emulate_long(const void *vin, void *vout, long long nvol)
     }
 }
 
+// The TRIP kernels (trip_kernels.cu k_trip; trip.cuh): three trips of a plane
+// item, two of a row item, every task of a trip before any of the next, as the
+// kernel's barriers order them.  Tickets, ring and dependency checks as
+// emulate_twopass.
+template <int N, typename T, int S, int G>
+static void emulate_trip(const void *vin, void *vout, long long nvol)
+{
+    using TR = Trip<N, T, G>;
+    using TG = TwoPassGeom<N, N, N, T, G>;
+    const T scale = S > 0 ? T(1) / T(TG::V) : T(1);
+    int lag = 0;
+    const int R = twopass_ring_size(TG::NA, TG::NB, 7, &lag);
+    std::vector<cx<T>> smv(TR::SM_ELEMS), ringbuf;
+    cx<T> *ring = aligned_ring(ringbuf, (long long)R * TG::V);
+    cx<T> *sm = smv.data();
+    cx<T> tw[TR::TW];
+    for (int e = 0; e < TR::TW; ++e) tw[e] = TR::tw_entry(e);
+    const cx<T> *in = (const cx<T> *)vin;
+    cx<T> *out = (cx<T> *)vout;
+    const long long total = (long long)(TG::NA + TG::NB) * nvol;
+    std::vector<long long> cnt_plane(R, 0), cnt_row(R, 0);
+    auto load = [](const cx<T> *p) { return *p; };
+    auto store = [](cx<T> *p, cx<T> v) { *p = v; };
+    for (long long tk = 0; tk < total; ++tk) {
+        const TwoPassItem it = twopass_decode(tk, nvol, TG::NA, TG::NB, lag);
+        const int slot = (int)(it.vol % R);
+        const long long round = it.vol / R;
+        cx<T> *sv = ring + slot * TG::V;
+        if (it.plane ? cnt_row[slot] < TG::NB * round : cnt_plane[slot] < TG::NA * (round + 1))
+            g_twopass_violations++;
+        (it.plane ? cnt_plane : cnt_row)[slot]++;
+        for (auto &e : smv) e = {T(12345.0), T(-6789.0)};
+        if (it.plane) {
+            const long long p0 = (long long)it.j * G * TR::PLANE;
+            for (int t = 0; t < TR::T1; ++t) {
+                cx<T> v[TR::A];
+                TR::trip1_load(in + it.vol * TG::V + p0, t, v, load);
+                TR::template trip1_store<S>(sm, t, v);
+            }
+            for (int t = 0; t < TR::T2; ++t) TR::template trip2<S>(sm, tw, t);
+            for (int t = 0; t < TR::T3; ++t) TR::template trip3<S>(sm, sv + p0, t, store);
+        } else {
+            const long long r0 = (long long)it.j * G * N;
+            for (int t = 0; t < TR::R1; ++t) {
+                cx<T> v[TR::A];
+                TR::row1_load(sv + r0, t, v, load);
+                TR::template row1_store<S>(sm, t, v);
+            }
+            poison_discarded_rows<TG>(sv, it.j);
+            for (int t = 0; t < TR::R2; ++t)
+                TR::template row2<S>(sm, tw, out + it.vol * TG::V + r0, t, scale, store);
+        }
+    }
+}
+
 typedef void (*emu_fn)(const void *, void *, long long);
 
 #define EMU_TPR_(N0, N1, N2, G, A, XB)                                                       \
@@ -499,6 +555,9 @@ typedef void (*emu_fn)(const void *, void *, long long);
 #define EMU_LONG(N0, N1, N2, T, VPC, KT)                                                      \
     {N0, N1, N2, sizeof(T) == 8 ? 0 : 1, -1, 2000 + KT, VPC, &emulate_long<N0, N1, N2, T, -1, VPC, KT>}, \
     {N0, N1, N2, sizeof(T) == 8 ? 0 : 1, +1, 2000 + KT, VPC, &emulate_long<N0, N1, N2, T, +1, VPC, KT>}
+#define EMU_TRIP(N, T, G)                                                                     \
+    {N, N, N, sizeof(T) == 8 ? 0 : 1, -1, 800 + G, 1, &emulate_trip<N, T, -1, G>},               \
+    {N, N, N, sizeof(T) == 8 ? 0 : 1, +1, 800 + G, 1, &emulate_trip<N, T, +1, G>}
 #define EMU_TP(N0, N1, N2, T, G)                                                              \
     {N0, N1, N2, sizeof(T) == 8 ? 0 : 1, -1, 300 + G, 1,                                    \
      &emulate_twopass<N0, N1, N2, T, -1, G>},                                                \
@@ -551,6 +610,7 @@ static const EmuEntry kEmu[] = {
     EMU_TPR(36, 36, 36, 3), EMU_TPR(36, 36, 36, 2), EMU_TPR(36, 36, 36, 4), EMU_TPRQ(36, 36, 36, 3),
     EMU_TPRQ(36, 36, 36, 2), EMU_TPRQ(6, 9, 5, 3), EMU_TPRQF(3), EMU_TPRQF(2), EMU_TPRQF(4), EMU_TPST(LineCT64, 64, double), EMU_TPST(LineCT64, 64, float), EMU_TPST(LinePFA45, 45, double),
     EMU_TPR(6, 9, 5, 3),
+    EMU_TRIP(64, double, 1),
     EMU_REC(16, 16, 32, double, 33, 27, 8), EMU_REC(23, 23, 23, double, 23, 23, 12),
     EMU_REC(23, 23, 23, double, 23, 27, 12), EMU_REC(24, 24, 24, double, 25, 24, 8),
     EMU_REC(30, 30, 30, float, 30, 30, 10), EMU_REC(16, 16, 16, double, 17, 16, 8),

@@ -66,6 +66,7 @@ void register_tc_kernels(std::vector<KernelEntry> &out);       // tc_kernels.cu
 int tc_tables_upload();                                         // split-BF16 DFT matrices
 void register_cluster_kernels(std::vector<KernelEntry> &out);  // cluster_kernels.cu
 void register_twopass_kernels(std::vector<KernelEntry> &out);  // twopass_kernels.cu
+void register_trip_kernels(std::vector<KernelEntry> &out);     // trip_kernels.cu
 
 // TWOPASS ring geometry for a launch of `grid` CTAs: returns the ring size R
 // (scratch volumes) and sets *lag to D, the distance in steps between the

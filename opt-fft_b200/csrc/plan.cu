@@ -52,6 +52,7 @@ const std::vector<KernelEntry> &registry()
         register_tc_kernels(reg);
         register_kernels(reg);
         register_cluster_kernels(reg);
+        register_trip_kernels(reg);
         register_twopass_kernels(reg);
     });
     return reg;

@@ -111,6 +111,24 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
     return false;
 }
 
+// The same, bounded in time, for a phase that another thread completes only
+// after a wait of up to kCounterWaitNs of its own.
+__device__ __forceinline__ bool mbar_wait_timed(uint64_t *bar, uint32_t parity)
+{
+    if (mbar_try_wait(bar, parity)) return true;
+    const unsigned long long t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 2 * kCounterWaitNs)
+        if (mbar_try_wait(bar, parity)) return true;
+    return false;
+}
+
+// Barrier among the `threads` threads (whole warps) that use barrier `id` (1..15;
+// 0 is __syncthreads).
+__device__ __forceinline__ void named_barrier_sync(int id, int threads)
+{
+    asm volatile("barrier.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
 // Order this thread's generic-proxy shared-memory accesses before later
 // async-proxy (TMA) accesses of the same memory.
 __device__ __forceinline__ void fence_proxy_async_smem()
@@ -206,6 +224,26 @@ __device__ __forceinline__ void st_cg_hint(float2 *p, float2 v, uint64_t policy)
     asm volatile("st.global.cg.L2::cache_hint.v2.f32 [%0], {%1, %2}, %3;" ::"l"(p), "f"(v.x), "f"(v.y),
                  "l"(policy)
                  : "memory");
+}
+
+// Loads of one complex value of data that this launch only reads, past L1, with
+// an L2 cache policy.
+__device__ __forceinline__ double2 ld_nc_hint(const double2 *p, uint64_t policy)
+{
+    double2 v;
+    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;"
+                 : "=d"(v.x), "=d"(v.y)
+                 : "l"(p), "l"(policy));
+    return v;
+}
+
+__device__ __forceinline__ float2 ld_nc_hint(const float2 *p, uint64_t policy)
+{
+    float2 v;
+    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;"
+                 : "=f"(v.x), "=f"(v.y)
+                 : "l"(p), "l"(policy));
+    return v;
 }
 
 // Drop the 128-byte L2 line at p (128-byte aligned) without writing it back;

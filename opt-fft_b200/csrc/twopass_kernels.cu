@@ -27,21 +27,9 @@
 #include "splitline.cuh"
 #include "staged.cuh"
 #include "twopass.cuh"
+#include "twopass_dev.cuh"
 
 namespace fft3d {
-
-// Every thread: drop from L2, without a write-back, the scratch lines whose
-// rows row item j has read for the last time (twopass_row_line).  A barrier
-// must follow before the slot is released to the next volume's plane items.
-template <class TG>
-__device__ __forceinline__ void twopass_discard_rows(const void *slot, int j, int tid, int nt)
-{
-    constexpr int NQ = TG::YG::N0 * twopass_row_lines_per_plane<TG>();
-    for (int q = tid; q < NQ; q += nt) {
-        uintptr_t line;
-        if (twopass_row_line<TG>(slot, j, q, &line)) discard_l2_line(line);
-    }
-}
 
 template <typename T>
 __device__ __forceinline__ cx<T> ld_l2(const cx<T> *p)
@@ -172,19 +160,7 @@ __global__ void __launch_bounds__(NT, MINB)
         report_error(err, DEV_ERR_DEP_TIMEOUT);
         atomicExch(&ctl->abort, 1u);
     }
-    // The last CTA to leave clears the control block for the next launch.
-    if (tid == 0) {
-        __threadfence();
-        const unsigned prev = atomicAdd(&ctl->done, 1u);
-        if (prev == gridDim.x - 1) {
-            __threadfence();  // every other CTA's updates of the block precede the reset
-            ctl->ticket = 0ull;
-            for (int i = 0; i < 2 * TWOPASS_RMAX; ++i) ctl->cnt[i] = 0u;
-            ctl->abort = 0u;
-            __threadfence();
-            ctl->done = 0u;
-        }
-    }
+    twopass_leave(ctl, tid);
 }
 
 // Pipelined TWOPASS (complex double): two shared-memory stages per CTA; while
@@ -318,18 +294,7 @@ __global__ void __launch_bounds__(NT, MINB)
         report_error(err, DEV_ERR_DEP_TIMEOUT);
         atomicExch(&ctl->abort, 1u);
     }
-    if (tid == 0) {
-        __threadfence();
-        const unsigned prev = atomicAdd(&ctl->done, 1u);
-        if (prev == gridDim.x - 1) {
-            __threadfence();
-            ctl->ticket = 0ull;
-            for (int i = 0; i < 2 * TWOPASS_RMAX; ++i) ctl->cnt[i] = 0u;
-            ctl->abort = 0u;
-            __threadfence();
-            ctl->done = 0u;
-        }
-    }
+    twopass_leave(ctl, tid);
 }
 
 // TWOPASS with lean item control (complex double, row-major layouts).  Thread
@@ -500,19 +465,7 @@ __global__ void __launch_bounds__(NT, MINB)
         report_error(err, DEV_ERR_DEP_TIMEOUT);
         atomicExch(&ctl->abort, 1u);
     }
-    // The last CTA to leave clears the control block for the next launch.
-    if (tid == 0) {
-        __threadfence();
-        const unsigned prev = atomicAdd(&ctl->done, 1u);
-        if (prev == gridDim.x - 1) {
-            __threadfence();
-            ctl->ticket = 0ull;
-            for (int i = 0; i < 2 * TWOPASS_RMAX; ++i) ctl->cnt[i] = 0u;
-            ctl->abort = 0u;
-            __threadfence();
-            ctl->done = 0u;
-        }
-    }
+    twopass_leave(ctl, tid);
 }
 
 // TWOPASS for N^3 complex double with every line split over P lanes of a warp
@@ -671,18 +624,7 @@ __global__ void __launch_bounds__(NT, MINB)
         report_error(err, DEV_ERR_DEP_TIMEOUT);
         atomicExch(&ctl->abort, 1u);
     }
-    if (tid == 0) {
-        __threadfence();
-        const unsigned prev = atomicAdd(&ctl->done, 1u);
-        if (prev == gridDim.x - 1) {
-            __threadfence();
-            ctl->ticket = 0ull;
-            for (int i = 0; i < 2 * TWOPASS_RMAX; ++i) ctl->cnt[i] = 0u;
-            ctl->abort = 0u;
-            __threadfence();
-            ctl->done = 0u;
-        }
-    }
+    twopass_leave(ctl, tid);
 }
 
 // TWOPASS for N^3 with every line split into two thread-level stages
@@ -833,19 +775,7 @@ __global__ void __launch_bounds__(NT, MINB)
         report_error(err, DEV_ERR_DEP_TIMEOUT);
         atomicExch(&ctl->abort, 1u);
     }
-    // The last CTA to leave clears the control block for the next launch.
-    if (tid == 0) {
-        __threadfence();
-        const unsigned prev = atomicAdd(&ctl->done, 1u);
-        if (prev == gridDim.x - 1) {
-            __threadfence();
-            ctl->ticket = 0ull;
-            for (int i = 0; i < 2 * TWOPASS_RMAX; ++i) ctl->cnt[i] = 0u;
-            ctl->abort = 0u;
-            __threadfence();
-            ctl->done = 0u;
-        }
-    }
+    twopass_leave(ctl, tid);
 }
 
 int twopass_ring(const KernelEntry &e, long long grid, int *lag)
