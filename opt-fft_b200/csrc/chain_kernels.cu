@@ -18,6 +18,7 @@
 
 #include "../../include/fft3d_b200.h"
 #include "internal.h"
+#include "ptx.cuh"
 #include "volume.cuh"
 
 namespace fft3d {
@@ -56,12 +57,92 @@ __global__ void __launch_bounds__(NT, 1)
     }
 }
 
+// The same chain with a volume spread over a cluster of CL CTAs, for batches that
+// leave SMs idle: CTA r holds planes [first(r), first(r + 1)) and transforms
+// their z and y lines; the x lines are divided among the CTAs, their points read
+// from and written back to the planes' owners through distributed shared memory.
+// A step is two cluster barriers longer and its passes CL times shorter: what
+// bounds a step of one CTA a volume is the FP64 pipe of one SM, with 3 of its
+// warps on one quarter and 2 on another.  Four CTAs measured, us a step at 32
+// volumes, one CTA a volume and a cluster: 17^3 c128 4.18 / 3.09, 24^3 c128 8.22 /
+// 5.21, 17^3 c64 2.62 / 2.11, 24^3 c64 3.70 / 3.31.  The smaller cubes lose (16^3
+// c128 2.23 / 2.4, c64 1.20 / 1.5; 12^3 c128 1.36 / 1.6): a few warps a CTA wait for
+// one another's latencies and the barriers.
+template <int N0, int CL>
+struct ChainSlabs {
+    FFT_HD static constexpr int first(int r) { return r * N0 / CL; }
+    FFT_HD static constexpr int owner(int x)
+    {
+        int r = 0;
+        while (first(r + 1) <= x) ++r;
+        return r;
+    }
+    static constexpr int MOST = (N0 + CL - 1) / CL;  // planes of the largest slab
+};
+
+template <class G, int ALG, int EPI, int CL, int NT>
+__global__ void __launch_bounds__(NT, 1)
+    k_chain_cluster(const cx<typename G::T> *__restrict__ x0, cx<typename G::T> *__restrict__ out,
+                    const cx<typename G::T> *__restrict__ cmap, long long nvol, long long steps,
+                    typename G::T uscale)
+{
+    using T = typename G::T;
+    using SL = ChainSlabs<G::N0, CL>;
+    constexpr int N1 = G::N1, N2 = G::N2, LPC = (N1 * N2 + CL - 1) / CL;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    cx<T> *sm = reinterpret_cast<cx<T> *>(smraw);
+    const int tid = threadIdx.x, rank = (int)cluster_rank();
+    const int xb = SL::first(rank), np = SL::first(rank + 1) - xb;
+    const long long e0 = (long long)(blockIdx.x / CL) * G::V;  // the grid holds whole clusters: < nvol
+    const long long p0 = e0 + (long long)xb * N1 * N2;
+    (void)nvol;
+    uint32_t at[CL];
+#pragma unroll
+    for (int r = 0; r < CL; ++r) at[r] = mapa_u32(sm, (uint32_t)r);
+    for (int g = tid; g < np * N1 * N2; g += NT) sm[G::off(g / N2, g % N2)] = load_in(x0 + p0 + g);
+    __syncthreads();
+    const int l0 = rank * LPC, l1 = l0 + LPC < N1 * N2 ? l0 + LPC : N1 * N2;
+    for (long long s = 0; s < steps; ++s) {
+        for (int r = tid; r < np * N1; r += NT) pass_z<G, -1, ALG>(sm, r);
+        __syncthreads();
+        for (int l = tid; l < np * N2; l += NT) pass_y<G, -1, ALG>(sm, l);
+        cluster_sync_hw();
+        for (int l = l0 + tid; l < l1; l += NT) {
+            const int y = l / N2, z = l % N2;
+            cx<T> v[G::N0];
+#pragma unroll
+            for (int x = 0; x < G::N0; ++x) {
+                const int o = SL::owner(x);
+                v[x] = ld_dsmem<T>(at[o] + (uint32_t)(G::off((x - SL::first(o)) * N1 + y, z) * G::EB));
+            }
+            dft<G::N0, -1, T, ALG>(v);
+#pragma unroll
+            for (int x = 0; x < G::N0; ++x) {
+                const int o = SL::owner(x);
+                st_dsmem<T>(at[o] + (uint32_t)(G::off((x - SL::first(o)) * N1 + y, z) * G::EB),
+                            chain_epilogue<EPI>(v[x], cmap, e0 + l + (long long)x * (N1 * N2), uscale));
+            }
+        }
+        cluster_sync_hw();
+    }
+    for (int g = tid; g < np * N1 * N2; g += NT) store_out(out + p0 + g, sm[G::off(g / N2, g % N2)]);
+}
+
 struct ChainEntry {
     int n0, n1, n2, precision, epi, vpc, threads, smem;
     const void *func;
+    // the cluster form: CTAs a volume (0: none), threads and shared memory a CTA
+    int cl, cl_threads, cl_smem;
+    const void *cl_func;
 };
 
-template <int N0, int N1, int N2, typename T, int EPI, int VPC, int NT>
+// A cluster CTA asks for more than half of an SM's shared memory, so that no two
+// share an SM: at 37 clusters of 17^3 the last ones did, and a step took 3.9 us.
+// chain_clusters() then counts the clusters that fit the device at once, and a
+// larger batch takes one CTA a volume.
+constexpr int CHAIN_CLUSTER_SMEM = 116 * 1024;
+
+template <int N0, int N1, int N2, typename T, int EPI, int VPC, int NT, int CL>
 static void add_chain(std::vector<ChainEntry> &out)
 {
     using G = Geom<N0, N1, N2, T>;
@@ -75,30 +156,42 @@ static void add_chain(std::vector<ChainEntry> &out)
     e.threads = NT;
     e.smem = VPC * G::PV * G::EB;
     e.func = (const void *)&k_chain<G, ALG_DEFAULT, EPI, VPC, NT>;
+    e.cl = CL;
+    e.cl_threads = e.cl_smem = 0;
+    e.cl_func = nullptr;
+    if constexpr (CL > 0) {
+        constexpr int MOST = ChainSlabs<N0, CL>::MOST;
+        constexpr int LINES = MOST * (N1 > N2 ? N1 : N2);
+        constexpr int CNT = (LINES + 31) / 32 * 32;
+        e.cl_threads = CNT;
+        // more than half of an SM's shared memory: one CTA an SM
+        e.cl_smem = MOST * N1 * G::P2 * G::EB > CHAIN_CLUSTER_SMEM ? MOST * N1 * G::P2 * G::EB : CHAIN_CLUSTER_SMEM;
+        e.cl_func = (const void *)&k_chain_cluster<G, ALG_DEFAULT, EPI, CL, CNT>;
+    }
     out.push_back(e);
 }
 
-#define FFT3D_CHAIN(N0, N1, N2, T, VPC, NT)                 \
-    add_chain<N0, N1, N2, T, EPI_UNITARY, VPC, NT>(out);    \
-    add_chain<N0, N1, N2, T, EPI_MAP, VPC, NT>(out)
+#define FFT3D_CHAIN(N0, N1, N2, T, VPC, NT, CL)             \
+    add_chain<N0, N1, N2, T, EPI_UNITARY, VPC, NT, CL>(out); \
+    add_chain<N0, N1, N2, T, EPI_MAP, VPC, NT, CL>(out)
 
 static std::vector<ChainEntry> build_chain_registry()
 {
     std::vector<ChainEntry> out;
     {
         // one volume group per CTA; small VPC keeps many CTAs busy for small batches
-        FFT3D_CHAIN(6, 6, 6, double, 1, 64);
-        FFT3D_CHAIN(8, 8, 8, double, 1, 64);
-        FFT3D_CHAIN(12, 12, 12, double, 1, 160);
-        FFT3D_CHAIN(16, 16, 16, double, 1, 256);
-        FFT3D_CHAIN(17, 17, 17, double, 1, 320);
-        FFT3D_CHAIN(24, 24, 24, double, 1, 288);
-        FFT3D_CHAIN(6, 6, 6, float, 1, 64);
-        FFT3D_CHAIN(8, 8, 8, float, 1, 64);
-        FFT3D_CHAIN(12, 12, 12, float, 1, 160);
-        FFT3D_CHAIN(16, 16, 16, float, 1, 256);
-        FFT3D_CHAIN(17, 17, 17, float, 1, 320);
-        FFT3D_CHAIN(24, 24, 24, float, 1, 576);
+        FFT3D_CHAIN(6, 6, 6, double, 1, 64, 0);
+        FFT3D_CHAIN(8, 8, 8, double, 1, 64, 0);
+        FFT3D_CHAIN(12, 12, 12, double, 1, 160, 0);
+        FFT3D_CHAIN(16, 16, 16, double, 1, 256, 0);
+        FFT3D_CHAIN(17, 17, 17, double, 1, 320, 4);
+        FFT3D_CHAIN(24, 24, 24, double, 1, 288, 4);
+        FFT3D_CHAIN(6, 6, 6, float, 1, 64, 0);
+        FFT3D_CHAIN(8, 8, 8, float, 1, 64, 0);
+        FFT3D_CHAIN(12, 12, 12, float, 1, 160, 0);
+        FFT3D_CHAIN(16, 16, 16, float, 1, 256, 0);
+        FFT3D_CHAIN(17, 17, 17, float, 1, 320, 4);
+        FFT3D_CHAIN(24, 24, 24, float, 1, 576, 4);
     }
     return out;
 }
@@ -113,12 +206,36 @@ static const std::vector<ChainEntry> &chain_registry()
 
 using namespace fft3d;
 
+// Clusters of e's cluster form that are resident at once, one CTA an SM (0: it
+// cannot run).
+static int chain_clusters(const ChainEntry &e)
+{
+    int n = 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)e.cl);
+    cfg.blockDim = dim3(e.cl_threads);
+    cfg.dynamicSmemBytes = (size_t)e.cl_smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)e.cl;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(e.cl_func, cudaFuncAttributeMaxDynamicSharedMemorySize, e.cl_smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, e.cl_func, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+
 struct fft3d_b200_chain {
     int device;
     int n0, n1, n2, precision, kind;
     long long batch;
     const void *cmap;
     const ChainEntry *e;
+    bool cluster;
     double uscale;
 };
 
@@ -142,6 +259,7 @@ extern "C" int fft3d_b200_chain_create(int n0, int n1, int n2, long long batch, 
     if (device < 0) device = prev < 0 ? 0 : prev;
     if (cudaSetDevice(device) != cudaSuccess) return FFT3D_B200_ERR_CUDA;
     int st = ensure_device_tables(device);
+    const bool cluster = st == FFT3D_B200_OK && e->cl > 0 && batch <= chain_clusters(*e);
     if (st == FFT3D_B200_OK &&
         cudaFuncSetAttribute(e->func, cudaFuncAttributeMaxDynamicSharedMemorySize, e->smem) !=
             cudaSuccess) {
@@ -160,6 +278,7 @@ extern "C" int fft3d_b200_chain_create(int n0, int n1, int n2, long long batch, 
     c->batch = batch;
     c->cmap = d_c;
     c->e = e;
+    c->cluster = cluster;
     c->uscale = 1.0 / std::sqrt((double)n0 * n1 * n2);
     *out = c;
     return FFT3D_B200_OK;
@@ -174,23 +293,35 @@ extern "C" int fft3d_b200_chain_run(fft3d_b200_chain *c, const void *d_x0, void 
     const size_t eb = (size_t)element_bytes(c->precision);
     if (((uintptr_t)d_x0 % eb) || ((uintptr_t)d_out % eb)) return FFT3D_B200_ERR_ALIGN;
     const ChainEntry &e = *c->e;
-    const long long grid = (c->batch + e.vpc - 1) / e.vpc;
+    const long long grid = c->cluster ? c->batch * e.cl : (c->batch + e.vpc - 1) / e.vpc;
     if (grid > 0x7fffffffLL) return FFT3D_B200_ERR_INVALID;
     long long nvol = c->batch;
     const void *cm = c->cmap;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(c->cluster ? e.cl_threads : e.threads);
+    cfg.dynamicSmemBytes = (size_t)(c->cluster ? e.cl_smem : e.smem);
+    cfg.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute attr[1];
+    if (c->cluster) {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)e.cl;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    const void *func = c->cluster ? e.cl_func : e.func;
     cudaError_t err;
     if (c->precision == FFT3D_B200_C128) {
         double us = c->uscale;
         void *args[] = {(void *)&d_x0, (void *)&d_out, (void *)&cm, (void *)&nvol, (void *)&steps,
                         (void *)&us};
-        err = cudaLaunchKernel(e.func, dim3((unsigned)grid), dim3(e.threads), args, (size_t)e.smem,
-                               (cudaStream_t)stream);
+        err = cudaLaunchKernelExC(&cfg, func, args);
     } else {
         float us = (float)c->uscale;
         void *args[] = {(void *)&d_x0, (void *)&d_out, (void *)&cm, (void *)&nvol, (void *)&steps,
                         (void *)&us};
-        err = cudaLaunchKernel(e.func, dim3((unsigned)grid), dim3(e.threads), args, (size_t)e.smem,
-                               (cudaStream_t)stream);
+        err = cudaLaunchKernelExC(&cfg, func, args);
     }
     return err == cudaSuccess ? FFT3D_B200_OK : FFT3D_B200_ERR_CUDA;
 }

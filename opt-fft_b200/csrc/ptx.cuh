@@ -9,6 +9,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "codelets.cuh"
+
 namespace fft3d {
 
 // Error codes written to a plan's device error word (first writer wins).
@@ -346,6 +348,28 @@ __device__ __forceinline__ float2 ld_dsmem_f32x2(uint32_t addr)
     asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr)
                  : "memory");
     return v;
+}
+
+// One complex value from, and to, another CTA's shared memory.
+template <typename T>
+__device__ __forceinline__ cx<T> ld_dsmem(uint32_t addr)
+{
+    if constexpr (sizeof(T) == 8) {
+        const double2 v = ld_dsmem_f64x2(addr);
+        return {v.x, v.y};
+    } else {
+        const float2 v = ld_dsmem_f32x2(addr);
+        return {v.x, v.y};
+    }
+}
+
+template <typename T>
+__device__ __forceinline__ void st_dsmem(uint32_t addr, cx<T> v)
+{
+    if constexpr (sizeof(T) == 8)
+        asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(addr), "d"(v.re), "d"(v.im) : "memory");
+    else
+        asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(v.re), "f"(v.im) : "memory");
 }
 
 // Record the first device-side error of a launch.
