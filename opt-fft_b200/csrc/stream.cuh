@@ -161,14 +161,18 @@ __global__ void __launch_bounds__(NT, MINB)
         const long long v0 = phys(item) * VPC;
         const int nv = (int)((nvol - v0) < VPC ? (nvol - v0) : VPC);
         cx<T> *sm = stage(cur);
-        for (int r = tid; r < nv * G::ROWS; r += NT) pass_z<G, S, ALG>(sm, r);
+        // an axis of length 1 has no pass (but for x, which scales the inverse)
+        if constexpr (G::N2 > 1)
+            for (int r = tid; r < nv * G::ROWS; r += NT) pass_z<G, S, ALG>(sm, r);
         if constexpr (BST)  // the stage refilled next held the previous item: its store has read it
             if (tid == 0) bulk_wait_read<0>();
-        __syncthreads();
+        if constexpr (BST || G::N2 > 1) __syncthreads();
         if constexpr (BST)
             if (ahead < nitems) issue(ahead, (k + NSTAGE - 1) % NSTAGE);
-        for (int l = tid; l < nv * G::N0 * G::N2; l += NT) pass_y<G, S, ALG>(sm, l);
-        __syncthreads();
+        if constexpr (G::N1 > 1) {
+            for (int l = tid; l < nv * G::N0 * G::N2; l += NT) pass_y<G, S, ALG>(sm, l);
+            __syncthreads();
+        }
         cx<T> *gout = out + v0 * G::V;
         if constexpr (BST) {
             // x pass in place, then one bulk store of the group (plain L2 policy:
@@ -220,14 +224,14 @@ __global__ void __launch_bounds__(NT, MINB)
 
 template <int N0, int N1, int N2, typename T, int S, int ALG, int VPC, int NT, int NSTAGE,
           int MINB, bool BST = false>
-static void add_stream(std::vector<KernelEntry> &out, const char *name)
+static void add_stream(std::vector<KernelEntry> &out, const char *name, int n0 = N0, int n1 = N1, int n2 = N2)
 {
     using G = Geom<N0, N1, N2, T>;
     constexpr int LOADER = (G::POL == 0) ? LOADER_BULK : LOADER_ASYNC;
     KernelEntry e;
-    e.n0 = N0;
-    e.n1 = N1;
-    e.n2 = N2;
+    e.n0 = n0;
+    e.n1 = n1;
+    e.n2 = n2;
     e.precision = sizeof(T) == 8 ? FFT3D_B200_C128 : FFT3D_B200_C64;
     e.sign = S;
     e.family = FAM_STREAM;
@@ -256,5 +260,13 @@ static void add_stream(std::vector<KernelEntry> &out, const char *name)
     add_stream<N0, N1, N2, T, +1, ALG, VPC, NT, NST, MINB, true>(                                 \
         out, "stream " #N0 "x" #N1 "x" #N2 " " #T " alg" #ALG " vpc" #VPC " nt" #NT " st" #NST   \
              " minb" #MINB " bst")
+
+// N0 x N1 x 1 volumes as 1 x N0 x N1 ones, the same points in the same order: their
+// rows of one point each would put the lanes of the y pass on one bank.
+#define FFT3D_STREAM_FLAT(N0, N1, T, VPC, NT, NST, MINB)                                          \
+    add_stream<1, N0, N1, T, -1, 0, VPC, NT, NST, MINB>(                                          \
+        out, "stream " #N0 "x" #N1 "x1 " #T " flat vpc" #VPC " nt" #NT " st" #NST " minb" #MINB, N0, N1, 1); \
+    add_stream<1, N0, N1, T, +1, 0, VPC, NT, NST, MINB>(                                          \
+        out, "stream " #N0 "x" #N1 "x1 " #T " flat vpc" #VPC " nt" #NT " st" #NST " minb" #MINB, N0, N1, 1)
 
 }  // namespace fft3d

@@ -9,7 +9,8 @@
 // on B200 over 96 MB (floor 30 us at 6.65 TB/s; a device copy takes 34.4 us),
 // VOLUME against STREAM: 9x25x7 c128 115 / 36.8 us, 11x4x9 81.9 / 35.9, 25x4x3
 // 82.4 / 37.0, 7x11x13 63.8 / 36.0, 15^3 59.9 / 37.7, 24x18x12 73.8 / 50.5,
-// 1x1x16 c64 125 / 33.8, 9x25x7 c64 95.4 / 37.0, 7x11x13 c64 68.5 / 38.1.  Of some
+// 1x1x16 c64 125 / 33.8, 9x25x7 c64 95.4 / 37.0, 7x11x13 c64 68.5 / 38.1, 1^3 102 /
+// 33.5, 8x8x1 (as 1x8x8) c128 66.9 / 35.7 and c64 48.4 / 39.0.  Of some
 // 900 shapes swept (2-4 stages, 1-8 CTAs an SM, register or bulk stores) the
 // fastest of each extent is kept, and a second one with smaller items where that
 // costs under 7%, for batches that the larger items would leave on few SMs.  The
@@ -22,6 +23,7 @@ namespace fft3d {
 void register_stream_odd_kernels(std::vector<KernelEntry> &out)
 {
     // complex double
+    FFT3D_STREAM_BST(1, 1, 1, double, 0, 1024, 256, 2, 4);
     FFT3D_STREAM(2, 2, 2, double, 0, 72, 160, 2, 8);
     FFT3D_STREAM(3, 3, 3, double, 0, 21, 192, 3, 4);
     FFT3D_STREAM_BST(5, 5, 5, double, 0, 9, 128, 3, 2);
@@ -41,8 +43,7 @@ void register_stream_odd_kernels(std::vector<KernelEntry> &out)
     FFT3D_STREAM(32, 8, 4, double, 0, 1, 64, 2, 3);
     FFT3D_STREAM(1, 8, 8, double, 0, 13, 128, 2, 4);
     FFT3D_STREAM_BST(8, 1, 8, double, 0, 13, 128, 4, 4);
-    FFT3D_STREAM_BST(8, 8, 1, double, 0, 37, 320, 3, 2);
-    FFT3D_STREAM(8, 8, 1, double, 0, 13, 128, 2, 4);
+    FFT3D_STREAM_FLAT(8, 8, double, 13, 128, 2, 4);
     FFT3D_STREAM_BST(49, 2, 2, double, 0, 8, 64, 2, 3);
     FFT3D_STREAM_BST(25, 4, 3, double, 0, 5, 64, 2, 4);
     FFT3D_STREAM(27, 2, 2, double, 0, 7, 64, 3, 2);
@@ -61,6 +62,7 @@ void register_stream_odd_kernels(std::vector<KernelEntry> &out)
     FFT3D_STREAM(20, 12, 6, double, 0, 1, 96, 2, 2);
     FFT3D_STREAM_BST(11, 4, 9, double, 0, 2, 64, 2, 4);
     // complex float
+    FFT3D_STREAM_BST(1, 1, 1, float, 0, 2048, 256, 2, 4);
     FFT3D_STREAM(2, 2, 2, float, 0, 148, 320, 2, 4);
     FFT3D_STREAM_BST(3, 3, 3, float, 0, 88, 512, 3, 2);
     FFT3D_STREAM(4, 4, 4, float, 0, 44, 512, 2, 2);
@@ -80,8 +82,7 @@ void register_stream_odd_kernels(std::vector<KernelEntry> &out)
     FFT3D_STREAM(17, 2, 2, float, 0, 17, 96, 2, 8);
     FFT3D_STREAM_BST(32, 8, 4, float, 0, 1, 64, 3, 2);
     FFT3D_STREAM(1, 8, 8, float, 0, 33, 160, 2, 3);
-    FFT3D_STREAM(8, 8, 1, float, 0, 56, 224, 2, 2);
-    FFT3D_STREAM_BST(8, 8, 1, float, 0, 18, 160, 3, 4);
+    FFT3D_STREAM_FLAT(8, 8, float, 33, 160, 2, 3);
     FFT3D_STREAM(49, 2, 2, float, 0, 6, 64, 2, 4);
     FFT3D_STREAM_BST(25, 4, 3, float, 0, 5, 64, 2, 8);
     FFT3D_STREAM_BST(27, 2, 2, float, 0, 10, 64, 2, 8);
