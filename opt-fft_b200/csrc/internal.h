@@ -86,6 +86,10 @@ cudaError_t launch_entry(const KernelEntry &e, const void *in, void *out, long l
                          double scale, cudaStream_t stream, int grid_limit, int *err,
                          void *work = nullptr);
 
+// Launch a kernel that begins with pdl_begin() (ptx.cuh) and uses no dynamic shared
+// memory, as launch_entry does: placed while the kernel before it drains.
+cudaError_t launch_dependent(const void *func, unsigned grid, int threads, void **args, cudaStream_t stream);
+
 // CTAs of `e` that fit on one SM (0 if it cannot launch); sets attributes on first use.
 int entry_occupancy(const KernelEntry &e, int device);
 

@@ -61,8 +61,7 @@ const std::vector<KernelEntry> &registry()
 // Programmatic dependent launch for every kernel started here (each calls
 // pdl_begin() before touching global memory): the CTAs of a launch are placed
 // while the previous kernel of the stream drains, and start work the moment it
-// completes.  FFT3D_B200_PDL=0 turns it off (plain stream order); the legacy
-// default stream always gets plain order.
+// completes.  FFT3D_B200_PDL=0 turns it off (plain stream order).
 static bool pdl_enabled()
 {
     static const bool on = [] {
@@ -89,7 +88,7 @@ static cudaError_t launch_ex(const KernelEntry &e, dim3 grid, void **args, cudaS
         attr[n].val.clusterDim.z = 1;
         ++n;
     }
-    if (pdl_enabled() && stream != nullptr && stream != cudaStreamLegacy) {
+    if (pdl_enabled()) {
         attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[n].val.programmaticStreamSerializationAllowed = 1;
         ++n;
@@ -97,6 +96,14 @@ static cudaError_t launch_ex(const KernelEntry &e, dim3 grid, void **args, cudaS
     cfg.attrs = attr;
     cfg.numAttrs = n;
     return cudaLaunchKernelExC(&cfg, e.func, args);
+}
+
+cudaError_t launch_dependent(const void *func, unsigned grid, int threads, void **args, cudaStream_t stream)
+{
+    KernelEntry e = {};
+    e.func = func;
+    e.threads = threads;
+    return launch_ex(e, dim3(grid), args, stream, 0);
 }
 
 cudaError_t launch_entry(const KernelEntry &e, const void *in, void *out, long long nvol,

@@ -8,13 +8,15 @@
 // volume, loads its T points (stride n0*n1*n2 -- consecutive threads read
 // consecutive addresses, so every load and store is coalesced), transforms them
 // in registers and stores them back.  Two HBM passes in all; the inverse scales
-// by 1/V in the 3D pass and by 1/T in the t pass.
+// by 1/V in the 3D pass and by 1/T in the t pass.  The t pass is launched as the
+// plans' kernels are, its CTAs placed while the 3D pass drains.
 #include <cuda_runtime.h>
 
 #include <string>
 
 #include "../../include/fft3d_b200.h"
 #include "internal.h"
+#include "ptx.cuh"
 #include "volume.cuh"
 
 namespace fft3d {
@@ -25,6 +27,7 @@ template <int TL, typename T, int S>
 __global__ void __launch_bounds__(TPASS_THREADS)
     k_tpass(cx<T> *__restrict__ data, long long vol_elems, long long nblocks_per_vol, T scale)
 {
+    pdl_begin();
     const long long b = blockIdx.x / nblocks_per_vol;
     const long long p = (blockIdx.x % nblocks_per_vol) * TPASS_THREADS + threadIdx.x;
     if (p >= vol_elems) return;
@@ -127,13 +130,11 @@ extern "C" int fft3d_b200_plan4d_execute(fft3d_b200_plan4d *p, const void *d_in,
     if (p->precision == FFT3D_B200_C128) {
         double sc = p->sign > 0 ? 1.0 / (double)p->nt : 1.0;
         void *args[] = {(void *)&d_out, (void *)&ve, (void *)&nbl, (void *)&sc};
-        e = cudaLaunchKernel(p->tk->func, dim3((unsigned)grid), dim3(TPASS_THREADS), args, 0,
-                             (cudaStream_t)stream);
+        e = launch_dependent(p->tk->func, (unsigned)grid, TPASS_THREADS, args, (cudaStream_t)stream);
     } else {
         float sc = p->sign > 0 ? 1.0f / (float)p->nt : 1.0f;
         void *args[] = {(void *)&d_out, (void *)&ve, (void *)&nbl, (void *)&sc};
-        e = cudaLaunchKernel(p->tk->func, dim3((unsigned)grid), dim3(TPASS_THREADS), args, 0,
-                             (cudaStream_t)stream);
+        e = launch_dependent(p->tk->func, (unsigned)grid, TPASS_THREADS, args, (cudaStream_t)stream);
     }
     return e == cudaSuccess ? FFT3D_B200_OK : FFT3D_B200_ERR_CUDA;
 }
