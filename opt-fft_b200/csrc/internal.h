@@ -73,6 +73,20 @@ void register_trip_kernels(std::vector<KernelEntry> &out);     // trip_kernels.c
 // plane items and the row items of one volume in the ticket order (D < R).
 int twopass_ring(const KernelEntry &e, long long grid, int *lag);
 
+// One volume of a list launch (cube_list_entry): its buffers and direction.
+struct TwoPassVol {
+    const void *in;
+    void *out;
+    int inverse;  // 0 forward, 1 inverse
+    int pad;
+};
+
+// The TWOPASS kernel of 36^3 over a list of volumes anywhere in memory, either
+// direction each: launch_entry with the device array of TwoPassVol as `in`, `out`
+// unused, the inverse's scale, and a workspace as for any TWOPASS entry.  Inputs
+// must be 16-byte aligned.
+const KernelEntry &cube_list_entry(int precision);
+
 // Device workspace a launch of `e` with up to `grid_limit` CTAs needs (0 for
 // every family but TWOPASS).  The control block must be zero before the first
 // launch; each launch leaves it zero again.

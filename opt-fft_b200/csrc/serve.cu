@@ -15,6 +15,11 @@
 // per-CTA scratch of the two-phase 36^3 route, allocated once at creation; the
 // hot loop allocates nothing on the device.
 //
+// 36^3 volumes, beyond one SM, take one SM about 100 us each in the persistent
+// kernel (complex double).  Where that is not hidden behind the rest of the batch,
+// the batch's cubes run before it in one TWOPASS launch over all requests' volumes
+// (cubes_by_list).
+//
 // A request whose extent is not one of the persistent kernel's kinds (any
 // other compiled extent) is launched on its own with its tuned kernel, on the
 // same stream as the batch (a scratch-ring kernel with the slot's workspace).
@@ -59,6 +64,7 @@ struct ServeReq {
     int kind, vpc, big;
     long long vol_elems;
     long long nitems;
+    bool cube;  // 36^3 that a list launch can take: 16-byte aligned input
 };
 
 struct ServeSlot {
@@ -91,6 +97,7 @@ struct fft3d_b200_server {
     size_t peak_used = 0;
     int grid = 0;
     long long scratch_per_cta = 0;
+    int cube_grid[2] = {0, 0};  // CTAs of a list launch, by precision
     std::vector<ServeSlot> slots;
     std::mutex mu;
     std::condition_variable cv;
@@ -155,6 +162,42 @@ static int launch_request(fft3d_b200_server *s, ServeSlot &slot, const ServeReq 
     return FFT3D_B200_OK;
 }
 
+// Whether the 36^3 volumes of a batch, n of one precision, are faster in a list
+// launch of their own than as items of the persistent kernel beside `other_bytes`
+// of other volumes.  Measured on B200, complex double / float: the list launch takes
+// 12 us + 0.48 / 0.26 us a volume; as an item, a volume holds one SM for 98 / 49 us
+// (0.66 / 0.33 us of the whole GPU), and the batch cannot end before its last one;
+// the other kinds move 2.3 TB/s.
+static bool cubes_by_list(int precision, long long n, double other_bytes)
+{
+    const bool c128 = precision == FFT3D_B200_C128;
+    const double other = other_bytes / 2.3e6;  // us
+    const double list = other + 12.0 + (c128 ? 0.48 : 0.26) * (double)n;
+    const double item = c128 ? 98.0 : 49.0;
+    const double items = std::max(item * (double)((n + 147) / 148), other + item / 148.0 * (double)n);
+    return n > 0 && list < items;
+}
+
+// The volumes of a slot's list launches lie at the end of its item buffers: a cube
+// counts as one item when requests are admitted, and is one or the other.
+static_assert(sizeof(TwoPassVol) <= sizeof(BatchItem) && alignof(TwoPassVol) <= alignof(BatchItem),
+              "a list's volumes in the place of items");
+
+// The slot's cubes of one precision in one TWOPASS launch, n volumes at item `first`
+// of its buffers.  Its workspace is the slot's scratch, which the
+// persistent kernel uses after it on the same stream; the control block in front is
+// the list launches' own, and each leaves it zero.
+static int launch_cubes(fft3d_b200_server *s, ServeSlot &slot, int precision, long long first, long long n)
+{
+    const KernelEntry &e = cube_list_entry(precision);
+    if (cudaMemcpyAsync(slot.d_items + first, slot.h_items + first, (size_t)n * sizeof(TwoPassVol),
+                        cudaMemcpyHostToDevice, slot.stream) != cudaSuccess ||
+        launch_entry(e, slot.d_items + first, nullptr, n, 1.0 / (36.0 * 36.0 * 36.0), slot.stream,
+                     s->cube_grid[precision == FFT3D_B200_C128 ? 0 : 1], slot.d_err, slot.d_scratch) != cudaSuccess)
+        return FFT3D_B200_ERR_CUDA;
+    return FFT3D_B200_OK;
+}
+
 // Launch every request of `slot` as one persistent batch (or, in plain mode,
 // one launch per request) and record the slot's completion event.
 static int launch_slot(fft3d_b200_server *s, ServeSlot &slot)
@@ -169,6 +212,33 @@ static int launch_slot(fft3d_b200_server *s, ServeSlot &slot)
         for (const ServeReq &r : slot.reqs)
             if (r.kind < 0)
                 if (const int e = launch_request(s, slot, r)) return e;
+        // the cubes: by a list launch, or as items of the batch
+        long long cubes[2] = {0, 0};
+        double other_bytes = 0;
+        for (const ServeReq &r : slot.reqs) {
+            if (r.cube) cubes[r.seg.precision == FFT3D_B200_C128 ? 0 : 1] += r.seg.batch;
+            else other_bytes += (double)r.bytes;
+        }
+        bool listed[2];
+        long long end = SERVE_MAX_ITEMS;  // of the item buffers not taken by volumes
+        for (int k = 0; k < 2; ++k) {
+            const int precision = k == 0 ? FFT3D_B200_C128 : FFT3D_B200_C64;
+            listed[k] = cubes_by_list(precision, cubes[k], other_bytes);
+            if (!listed[k]) continue;
+            end -= cubes[k];
+            TwoPassVol *vol = reinterpret_cast<TwoPassVol *>(slot.h_items + end);
+            for (const ServeReq &r : slot.reqs) {
+                if (!r.cube || r.seg.precision != precision) continue;
+                const size_t vb = (size_t)r.vol_elems * (size_t)element_bytes(precision);
+                for (long long v = 0; v < r.seg.batch; ++v)
+                    *vol++ = {(const char *)r.seg.in + v * vb, (char *)r.seg.out + v * vb,
+                              r.seg.direction == FFT3D_B200_BACKWARD ? 1 : 0, 0};
+            }
+            if (const int e = launch_cubes(s, slot, precision, end, cubes[k])) return e;
+        }
+        auto in_batch = [&](const ServeReq &r) {
+            return r.kind >= 0 && !(r.cube && listed[r.seg.precision == FFT3D_B200_C128 ? 0 : 1]);
+        };
         // descriptors: requests are segments; items largest first
         int nseg = (int)slot.reqs.size();
         std::vector<int> order(nseg);
@@ -191,8 +261,8 @@ static int launch_slot(fft3d_b200_server *s, ServeSlot &slot)
             d.nvol = r.seg.batch;
             d.kind = r.kind < 0 ? 0 : r.kind;
             d.pad = 0;
-            if (r.kind < 0) {
-                d.nvol = 0;  // launched on its own above; no item refers to it
+            if (!in_batch(r)) {
+                d.nvol = 0;  // launched above; no item refers to it
                 continue;
             }
             int so = 0;
@@ -203,7 +273,7 @@ static int launch_slot(fft3d_b200_server *s, ServeSlot &slot)
         for (int oi = 0; oi < nseg; ++oi) {
             const int i = order[oi];
             const ServeReq &r = slot.reqs[i];
-            if (r.kind < 0) continue;
+            if (!in_batch(r)) continue;
             for (long long v0 = 0; v0 < r.seg.batch; v0 += r.vpc) {
                 BatchItem &it = slot.h_items[n++];
                 it.kind = r.kind;
@@ -224,7 +294,7 @@ static int launch_slot(fft3d_b200_server *s, ServeSlot &slot)
         const BatchItem *items = slot.d_items;
         const BatchSeg *segs = slot.d_segs;
         unsigned int *ticket = slot.d_ticket;
-        unsigned char *scratch = slot.d_scratch;
+        unsigned char *scratch = slot.d_scratch + TWOPASS_CTL_BYTES;
         long long spc = s->scratch_per_cta;
         const unsigned char *so = slot.d_solo;
         int *err = slot.d_err;
@@ -391,6 +461,15 @@ extern "C" int fft3d_b200_server_create(size_t hbm_budget_bytes, int max_infligh
         return fail(FFT3D_B200_ERR_UNSUPPORTED);
     s->grid = occ * sms;
     s->scratch_per_cta = (long long)36 * 36 * 36 * 16;  // the largest two-phase volume
+    // a slot's scratch: the list launches' control block, then the larger of their
+    // ring and the persistent kernel's scratch volumes
+    size_t scratch_bytes = TWOPASS_CTL_BYTES + (size_t)s->scratch_per_cta * s->grid;
+    for (int k = 0; k < 2; ++k) {
+        const KernelEntry &e = cube_list_entry(k == 0 ? FFT3D_B200_C128 : FFT3D_B200_C64);
+        s->cube_grid[k] = entry_occupancy(e, device) * sms;
+        if (s->cube_grid[k] < 1) return fail(FFT3D_B200_ERR_UNSUPPORTED);
+        scratch_bytes = std::max(scratch_bytes, entry_workspace_bytes(e, s->cube_grid[k]));
+    }
     s->slots.resize((size_t)max_inflight);
     for (ServeSlot &slot : s->slots) {
         if (cudaStreamCreateWithFlags(&slot.stream, cudaStreamNonBlocking) != cudaSuccess ||
@@ -403,7 +482,8 @@ extern "C" int fft3d_b200_server_create(size_t hbm_budget_bytes, int max_infligh
                 cudaMalloc(&slot.d_segs, sizeof(BatchSeg) * SERVE_MAX_SEGS) != cudaSuccess ||
                 cudaMalloc(&slot.d_ticket, sizeof(unsigned int)) != cudaSuccess ||
                 cudaMalloc(&slot.d_solo, BATCH_NKINDS) != cudaSuccess ||
-                cudaMalloc(&slot.d_scratch, (size_t)s->scratch_per_cta * s->grid) != cudaSuccess ||
+                cudaMalloc(&slot.d_scratch, scratch_bytes) != cudaSuccess ||
+                cudaMemset(slot.d_scratch, 0, TWOPASS_CTL_BYTES) != cudaSuccess ||
                 cudaHostAlloc(&slot.h_items, sizeof(BatchItem) * SERVE_MAX_ITEMS, 0) != cudaSuccess ||
                 cudaHostAlloc(&slot.h_segs, sizeof(BatchSeg) * SERVE_MAX_SEGS, 0) != cudaSuccess)
                 return fail(FFT3D_B200_ERR_NOMEM);
@@ -437,6 +517,7 @@ static int server_submit_at(fft3d_b200_server *s, const fft3d_b200_segment *req,
         r.big = 0;
         r.vol_elems = (long long)q.n0 * q.n1 * q.n2;
     }
+    r.cube = r.kind >= 0 && q.n0 == 36 && q.n1 == 36 && q.n2 == 36 && (uintptr_t)q.in % 16 == 0;
     const size_t eb = (size_t)element_bytes(q.precision);
     r.bytes = 2 * (size_t)q.batch * (size_t)r.vol_elems * eb;
     if (((uintptr_t)q.in % eb) || ((uintptr_t)q.out % eb)) return FFT3D_B200_ERR_ALIGN;

@@ -314,8 +314,15 @@ __global__ void __launch_bounds__(NT, MINB)
 // ranges; no shared memory at all, "regs" in the name) or gather their rows by
 // bulk copies first (XBULK, "bulkqh").  HINT adds the L2 policies: input rows
 // evict_first, ring stores evict_last.
+// LIST: `in` is an array of TwoPassVol, one per volume -- the volumes lie anywhere,
+// each with a direction of its own (a batch of many requests' cubes in one launch).
+template <int S>
+struct SignC {
+    static constexpr int value = S;
+};
+
 template <int N0, int N1, int N2, int S, int G, int NT, int MINB, bool XBULK = false,
-          bool HINT = false, typename T = double, int PITCH = 0>
+          bool HINT = false, typename T = double, int PITCH = 0, bool LIST = false>
 __global__ void __launch_bounds__(NT, MINB)
     k_twopass_regs(const cx<T> *__restrict__ in, cx<T> *__restrict__ out, long long nvol, T scale,
                    int *err, unsigned char *work, int R, int D)
@@ -325,6 +332,7 @@ __global__ void __launch_bounds__(NT, MINB)
     using XG = typename TG::XG;
     using YG = typename TG::YG;
     static_assert(XG::POL != 2 && YG::POL != 2 && NT % 32 == 0, "row-major layouts, whole warps");
+    static_assert(!LIST || (XBULK && HINT), "list launches gather their rows by bulk copies");
     constexpr uint32_t ROW_BYTES = (uint32_t)(N2 * sizeof(cx<T>));
     static_assert(ROW_BYTES % 16 == 0 && (XG::P2 * XG::EB) % 16 == 0,
                   "bulk row copies: 16-byte rows at 16-byte aligned shared-memory starts");
@@ -378,11 +386,26 @@ __global__ void __launch_bounds__(NT, MINB)
         const TwoPassItem it = twopass_decode(s_t, nvol, TG::NA, TG::NB, D);
         const int slot = (int)(it.vol % R);
         cx<T> *sv = ring + (long long)slot * TG::V;
+        const cx<T> *vin = in + it.vol * TG::V;
+        cx<T> *vout = out + it.vol * TG::V;
+        bool inverse = S > 0;
+        if constexpr (LIST) {
+            const TwoPassVol v = reinterpret_cast<const TwoPassVol *>(in)[it.vol];
+            vin = reinterpret_cast<const cx<T> *>(v.in);
+            vout = reinterpret_cast<cx<T> *>(v.out);
+            inverse = v.inverse != 0;
+        }
+        // f(SignC<direction>): a list's directions are uniform over an item
+        auto in_direction = [&](auto f) {
+            if constexpr (!LIST) f(SignC<S>{});
+            else if (inverse) f(SignC<INV>{});
+            else f(SignC<FWD>{});
+        };
 
         if (it.plane) {
             // 1. G contiguous planes of the input, one bulk copy per row
             if (tid == 0) mbar_arrive_expect_tx(&s_bar, (uint32_t)XG::ROWS * ROW_BYTES);
-            const cx<T> *rows = in + it.vol * TG::V + (long long)it.j * G * N1 * N2;
+            const cx<T> *rows = vin + (long long)it.j * G * N1 * N2;
             for (int r = tid; r < XG::ROWS; r += NT) {
                 if constexpr (HINT)  // read once: do not displace the ring
                     bulk_g2s_hint(sm + XG::off(r, 0), rows + (long long)r * N2, ROW_BYTES, &s_bar, pol_first);
@@ -400,26 +423,25 @@ __global__ void __launch_bounds__(NT, MINB)
             __syncthreads();
             if (s_stop) break;
             // 2. z pass in shared memory
-            for (int r = tid; r < XG::ROWS; r += NT) pass_z<XG, S, ALG_DEFAULT>(sm, r);
+            in_direction([&](auto sign) {
+                for (int r = tid; r < XG::ROWS; r += NT) pass_z<XG, decltype(sign)::value, ALG_DEFAULT>(sm, r);
+            });
             __syncthreads();
             // 3. y pass into the scratch slot (its previous reader is done: checked in step 1)
             if constexpr (HINT) {
                 // ring lines stay in L2 (evict_last): a slot is rewritten in L2, not written back
-                for (int l = tid; l < G * N2; l += NT) {
-                    const int z = l % N2, g = l / N2;
-                    cx<T> v[N1];
+                in_direction([&](auto sign) {
+                    for (int l = tid; l < G * N2; l += NT) {
+                        const int z = l % N2, g = l / N2;
+                        cx<T> v[N1];
 #pragma unroll
-                    for (int j = 0; j < N1; ++j) v[j] = sm[XG::off(g * N1 + j, z)];
-                    dft<N1, S, T>(v);
-                    cx<T> *o = sv + (long long)(it.j * G + g) * N1 * N2 + z;
+                        for (int j = 0; j < N1; ++j) v[j] = sm[XG::off(g * N1 + j, z)];
+                        dft<N1, decltype(sign)::value, T>(v);
+                        cx<T> *o = sv + (long long)(it.j * G + g) * N1 * N2 + z;
 #pragma unroll
-                    for (int j = 0; j < N1; ++j) {
-                        if constexpr (sizeof(T) == 8)
-                            st_cg_hint(reinterpret_cast<double2 *>(o + j * N2), make_double2(v[j].re, v[j].im), pol_last);
-                        else
-                            st_cg_hint(reinterpret_cast<float2 *>(o + j * N2), make_float2(v[j].re, v[j].im), pol_last);
+                        for (int j = 0; j < N1; ++j) st_hint(o + j * N2, v[j], pol_last);
                     }
-                }
+                });
             } else {
                 for (int l = tid; l < G * N2; l += NT) pass_y_store_l2<XG, S>(sm, l, sv, it.j * G);
             }
@@ -444,14 +466,16 @@ __global__ void __launch_bounds__(NT, MINB)
             __syncthreads();
             if (tid == 0) red_release_gpu_add(&ctl->cnt[TWOPASS_RMAX + slot], 1u);
             // 2. x pass, straight to the output
-            for (int l = tid; l < G * N2; l += NT)
-                pass_x_slab<YG, S, N1>(sm, l, out + it.vol * TG::V, it.j * G, scale);
+            in_direction([&](auto sign) {
+                for (int l = tid; l < G * N2; l += NT)
+                    pass_x_slab<YG, decltype(sign)::value, N1>(sm, l, vout, it.j * G, scale);
+            });
             fence_proxy_async_smem();
             __syncthreads();
         } else {
             // x pass from the scratch slot (its plane items are done: checked above)
             for (int l = tid; l < G * N2; l += NT)
-                pass_x_load_l2<N0, N1, N2, S, T>(sv, l, out + it.vol * TG::V, it.j * G, scale);
+                pass_x_load_l2<N0, N1, N2, S, T>(sv, l, vout, it.j * G, scale);
             __syncthreads();  // every load of the slot has returned
             twopass_discard_rows<TG>(sv, it.j, tid, NT);
             __syncthreads();
@@ -850,7 +874,7 @@ static void add_twopass_pipe(std::vector<KernelEntry> &out, const char *name)
 }
 
 template <int N0, int N1, int N2, int S, int G, int NT, int MINB, bool XBULK = false,
-          bool HINT = false, typename T = double, int PITCH = 0>
+          bool HINT = false, typename T = double, int PITCH = 0, bool LIST = false>
 static void add_twopass_regs(std::vector<KernelEntry> &out, const char *name)
 {
     using TG = TwoPassGeom<N0, N1, N2, T, G, PITCH>;
@@ -867,7 +891,7 @@ static void add_twopass_regs(std::vector<KernelEntry> &out, const char *name)
     e.threads = NT;
     // plane items only, unless row items gather their rows into shared memory too
     e.smem = XBULK ? TG::SMEM : ((XG::PV * XG::EB) + 127) / 128 * 128;
-    e.func = (const void *)&k_twopass_regs<N0, N1, N2, S, G, NT, MINB, XBULK, HINT, T, PITCH>;
+    e.func = (const void *)&k_twopass_regs<N0, N1, N2, S, G, NT, MINB, XBULK, HINT, T, PITCH, LIST>;
     e.name = name;
     out.push_back(e);
 }
@@ -983,6 +1007,18 @@ void register_twopass_kernels(std::vector<KernelEntry> &out)
     FFT3D_TWOPASS_STAGED(LineCT64, 64, float, "ct", 256, 3);
     FFT3D_TWOPASS(64, 64, 64, float, 2, 128, 3);
     FFT3D_TWOPASS(64, 64, 64, float, 4, 256, 1);
+}
+
+// Not among the registry's variants: a list launch takes other arguments.
+const KernelEntry &cube_list_entry(int precision)
+{
+    static const std::vector<KernelEntry> entries = [] {
+        std::vector<KernelEntry> e;
+        add_twopass_regs<36, 36, 36, INV, 3, 128, 3, true, true, double, 0, true>(e, "list 36x36x36 double");
+        add_twopass_regs<36, 36, 36, INV, 3, 128, 5, true, true, float, 38, true>(e, "list 36x36x36 float");
+        return e;
+    }();
+    return entries[precision == FFT3D_B200_C128 ? 0 : 1];
 }
 
 }  // namespace fft3d
