@@ -34,6 +34,7 @@ __global__ void __launch_bounds__(NT, MINB)
     using T = typename RG::T;
     using G = typename RG::G;
     constexpr int N0 = G::N0, N1 = G::N1, N2 = G::N2, NP = RG::NP, C = RG::C;
+    static_assert((long long)G::V * G::EB % 16 == 0, "volumes stay aligned");
     static_assert(RG::RC * N2 <= NT, "one x line of a chunk per thread");
     extern __shared__ __align__(128) unsigned char smraw[];
     cx<T> *sm = reinterpret_cast<cx<T> *>(smraw);
@@ -42,6 +43,7 @@ __global__ void __launch_bounds__(NT, MINB)
     const int tid = threadIdx.x;
     const long long mine = (nvol - blockIdx.x + gridDim.x - 1) / gridDim.x;  // this CTA's volumes
     const uint64_t pol_first = l2_policy_evict_first();
+    const bool aligned = (uintptr_t)in % 16 == 0;  // V and the rows are multiples of 16 bytes
     for (int i = tid; i < NP * C; i += NT) mbar_init(&full[i], 1);
     if (tid == 0) s_abort = 0;
     fence_mbar_init();
@@ -55,8 +57,18 @@ __global__ void __launch_bounds__(NT, MINB)
         const int x = (int)(q % N0), s = (int)(q % NP), y = c * RG::RC + yy;
         uint64_t *bar = &full[s * C + c];
         const uint32_t rows = (uint32_t)RG::rows(c);
-        if (yy == 0) mbar_arrive_expect_tx(bar, rows * RG::ROW_BYTES);
         const cx<T> *src = in + (blockIdx.x + k * gridDim.x) * G::V + (x * N1 + y) * N2;
+        if constexpr (G::EB == 8) {
+            if (!aligned) {  // complex float off a 16-byte boundary: one thread copies the chunk
+                if (yy == 0) {
+                    for (int j = 0; j < (int)rows * N2; ++j)
+                        sm[G::off(s * N1 + y + j / N2, j % N2)] = load_in(src + j);
+                    mbar_arrive(bar);
+                }
+                return;
+            }
+        }
+        if (yy == 0) mbar_arrive_expect_tx(bar, rows * RG::ROW_BYTES);
         if constexpr (G::P2 == N2) {  // the chunk's rows are one range
             if (yy == 0) bulk_g2s_hint(sm + G::off(s * N1 + y, 0), src, rows * RG::ROW_BYTES, bar, pol_first);
         } else {
