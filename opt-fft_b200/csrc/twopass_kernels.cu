@@ -403,10 +403,14 @@ __global__ void __launch_bounds__(NT, MINB)
         };
 
         if (it.plane) {
-            // 1. G contiguous planes of the input, one bulk copy per row
-            if (tid == 0) mbar_arrive_expect_tx(&s_bar, (uint32_t)XG::ROWS * ROW_BYTES);
+            // 1. G contiguous planes of the input, one bulk copy per row (complex float off
+            //    a 16-byte boundary: element by element)
             const cx<T> *rows = vin + (long long)it.j * G * N1 * N2;
-            for (int r = tid; r < XG::ROWS; r += NT) {
+            const bool bulk = sizeof(T) == 8 || (uintptr_t)rows % 16 == 0;
+            if (!bulk)
+                for (int g = tid; g < TG::PLANE_ELEMS; g += NT) sm[XG::off(g / N2, g % N2)] = load_in(rows + g);
+            if (bulk && tid == 0) mbar_arrive_expect_tx(&s_bar, (uint32_t)XG::ROWS * ROW_BYTES);
+            for (int r = bulk ? tid : XG::ROWS; r < XG::ROWS; r += NT) {
                 if constexpr (HINT)  // read once: do not displace the ring
                     bulk_g2s_hint(sm + XG::off(r, 0), rows + (long long)r * N2, ROW_BYTES, &s_bar, pol_first);
                 else
@@ -419,7 +423,7 @@ __global__ void __launch_bounds__(NT, MINB)
                 if (target > 0 && !wait_counter_geq(&ctl->cnt[TWOPASS_RMAX + slot], target, &ctl->abort))
                     s_stop = 2;
             }
-            if (!wait_copies()) s_stop = 2;
+            if (bulk && !wait_copies()) s_stop = 2;
             __syncthreads();
             if (s_stop) break;
             // 2. z pass in shared memory
@@ -727,10 +731,14 @@ __global__ void __launch_bounds__(NT, MINB)
         cx<T> *sv = ring + (long long)slot * TG::V;
 
         if (it.plane) {
-            // 1. x-plane j of the input, one bulk copy per y-row (read once: evict_first)
-            if (tid == 0) mbar_arrive_expect_tx(&s_bar, (uint32_t)N * ROW_BYTES);
+            // 1. x-plane j of the input, one bulk copy per y-row (read once: evict_first;
+            //    complex float off a 16-byte boundary: element by element)
             const cx<T> *rows = in + it.vol * TG::V + (long long)it.j * PLANE;
-            for (int r = tid; r < N; r += NT)
+            const bool bulk = sizeof(T) == 8 || (uintptr_t)rows % 16 == 0;
+            if (!bulk)
+                for (int g = tid; g < PLANE; g += NT) sm[g / N * P + g % N] = load_in(rows + g);
+            if (bulk && tid == 0) mbar_arrive_expect_tx(&s_bar, (uint32_t)N * ROW_BYTES);
+            for (int r = bulk ? tid : N; r < N; r += NT)
                 bulk_g2s_hint(sm + r * P, rows + (long long)r * N, ROW_BYTES, &s_bar, pol_first);
             // while the rows are in flight: the slot's previous volume must have
             // been read out before this item's y pass stores into it
@@ -739,7 +747,7 @@ __global__ void __launch_bounds__(NT, MINB)
                 if (target > 0 && !wait_counter_geq(&ctl->cnt[TWOPASS_RMAX + slot], target, &ctl->abort))
                     s_stop = 2;
             }
-            if (!wait_copies()) s_stop = 2;
+            if (bulk && !wait_copies()) s_stop = 2;
             __syncthreads();
             if (s_stop) break;
             // 2. z pass along the rows, in place (rows end in Line::slot order)

@@ -48,22 +48,3 @@ def test_literal_factors_are_the_tables(hostcheck, n):
     hostcheck.hostcheck_literal_factors.argtypes = [ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p]
     assert hostcheck.hostcheck_literal_factors(n, lit.ctypes.data, tab.ctypes.data) == 0
     assert np.array_equal(lit, tab)
-
-
-@pytest.mark.gpu
-@pytest.mark.parametrize("offset", [0, 8])
-def test_complex64_inputs_off_16_bytes(offset):
-    """30^3 complex64 needs its buffers aligned to 8 bytes only; its rows are copied in bulk from 16."""
-    torch = pytest.importorskip("torch")
-    import fft3d_b200 as fb
-    shape, n = (30, 30, 30), 300  # some CTAs take three volumes
-    x = field(np.random.default_rng(30), (n,) + shape, dtype=np.complex64)
-    raw = [torch.zeros(x.nbytes + 16, dtype=torch.uint8, device="cuda") for _ in range(2)]
-    a, b = (r[offset:offset + x.nbytes].view(torch.complex64).view(x.shape) for r in raw)
-    a.copy_(torch.from_numpy(x))
-    variant = next(v for v in fb.variants(shape, fb.C64) if v.startswith("recycle"))
-    plan = fb.Plan(shape, n, fb.FORWARD, fb.C64, variant=variant)
-    plan.execute(a.data_ptr(), b.data_ptr())
-    plan.check()
-    err = oracle.rel_error_per_volume(b.cpu().numpy()[::23].astype(np.complex128), oracle.fft3d(x[::23].astype(np.complex128)))
-    assert err.max() < C64_TOL
