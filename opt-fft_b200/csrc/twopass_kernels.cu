@@ -999,13 +999,17 @@ void register_twopass_kernels(std::vector<KernelEntry> &out)
     FFT3D_TWOPASS_BULKQH_F(36, 36, 36, 3, 128, 5, 38);
     FFT3D_TWOPASS_BULKQH_F(36, 36, 36, 2, 96, 6, 38);
     FFT3D_TWOPASS_BULKQH_F(36, 36, 36, 4, 160, 3, 38);
+    // 30^3 complex double, as 36^3: element copies by all threads bound it (k_twopass, 96
+    // threads, four CTAs an SM).  Two planes an item leave room for six CTAs an SM at 170
+    // registers a thread: 233 volumes 63.4 us (85.5 before; three planes 66.1, one 69.1,
+    // seven CTAs 72), two volumes 12.6 (16.2), 485 volumes 117 (164); three planes an item
+    // win at 72 volumes, 30.8 us against 31.3 (36.8).
+    FFT3D_TWOPASS_BULKQH(30, 30, 30, 2, 64, 6);
+    FFT3D_TWOPASS_BULKQH(30, 30, 30, 3, 96, 4);
     // 45^3: complex double five planes per item; 45 = 5 x 9 staged lines
     FFT3D_TWOPASS_BULKQH(45, 45, 45, 5, 256, 1);
     FFT3D_TWOPASS_STAGED(LinePFA45, 45, double, "pfa", 128, 6);
     // 45^3 complex float (a 360-byte row cannot be a bulk copy): element copies
-    // 30^3 complex128 (446 KB a volume), a test geometry of the reference
-    FFT3D_TWOPASS(30, 30, 30, double, 3, 96, 4);
-    FFT3D_TWOPASS(30, 30, 30, double, 5, 160, 3);
     FFT3D_TWOPASS(45, 45, 45, float, 5, 256, 2);
     FFT3D_TWOPASS(45, 45, 45, float, 3, 160, 3);
     // 64^3: 64 = 8 x 8 staged lines, one plane or y-row per item
