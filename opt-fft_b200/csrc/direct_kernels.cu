@@ -161,9 +161,7 @@ void register_direct_kernels(std::vector<KernelEntry> &out)
     FFT3D_DIRECT(17, 17, 17, double, 0, 1, 320, 1);
     FFT3D_DIRECT(24, 24, 24, double, 0, 1, 288, 1);
     FFT3D_DIRECT(8, 8, 16, double, 0, 2, 256, 2);
-    FFT3D_DIRECT(16, 16, 32, double, 0, 1, 256, 1);
     // pipelined through registers
-    FFT3D_DIRECT_PIPE(16, 16, 32, double, 1, 256, 1);
     FFT3D_DIRECT_PIPE(16, 16, 16, double, 1, 256, 1);
     FFT3D_DIRECT_PIPE(17, 17, 17, double, 1, 320, 1);
     FFT3D_DIRECT_PIPE(12, 12, 12, double, 2, 288, 1);

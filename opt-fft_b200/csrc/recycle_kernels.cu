@@ -149,6 +149,8 @@ static void add_recycle(std::vector<KernelEntry> &out, const char *name)
 
 void register_recycle_kernels(std::vector<KernelEntry> &out)
 {
+    // 384 volumes 51.1 us; DIRECT, pipelined and plain, 60.9 and 73.2 (10.3 against 9.4 us for
+    // one volume, where VOLUME takes 8.2): not compiled for this extent any more
     FFT3D_RECYCLE(16, 16, 32, double, 0, 33, 27, 8, 256, 1);
     FFT3D_RECYCLE(23, 23, 23, double, 0, 23, 23, 12, 288, 1);
     FFT3D_RECYCLE(24, 24, 24, double, 0, 25, 24, 8, 192, 1);

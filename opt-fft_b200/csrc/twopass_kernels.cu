@@ -1012,9 +1012,8 @@ void register_twopass_kernels(std::vector<KernelEntry> &out)
     // 45^3 complex float (a 360-byte row cannot be a bulk copy): element copies
     FFT3D_TWOPASS(45, 45, 45, float, 5, 256, 2);
     FFT3D_TWOPASS(45, 45, 45, float, 3, 160, 3);
-    // 64^3: 64 = 8 x 8 staged lines, one plane or y-row per item
-    FFT3D_TWOPASS_STAGED(LineCT64, 64, double, "ct", 128, 3);
-    FFT3D_TWOPASS_STAGED(LineCT64, 64, double, "ct", 256, 3);
+    // 64^3 complex float: 64 = 8 x 8 staged lines, one plane or y-row per item (complex
+    // double is TRIP's: 15.0 us against 16.7 for one volume, 75 against 93 for 24)
     FFT3D_TWOPASS_STAGED(LineCT64, 64, float, "ct", 128, 6);
     FFT3D_TWOPASS_STAGED(LineCT64, 64, float, "ct", 256, 3);
     FFT3D_TWOPASS(64, 64, 64, float, 2, 128, 3);
