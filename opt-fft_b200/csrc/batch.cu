@@ -12,9 +12,12 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -118,11 +121,36 @@ struct fft3d_b200_batch {
     bool segments = false;
     std::vector<fft3d_b200_plan *> plans;  // one per segment (NULL for empty ones)
     std::vector<cudaStream_t> branch;
+    size_t width = 0;  // branches in use
     std::vector<cudaEvent_t> join;
     cudaEvent_t fork = nullptr;
     cudaGraph_t sgraph = nullptr;
     cudaGraphExec_t sexec = nullptr;
 };
+
+// What a race between the strategies found, kept per process for batches of the same
+// segments (up to the size class of their volume counts) as the autotuner keeps its
+// choices: a program that makes a batch for each set of buffers races once.
+struct BatchChoice {
+    size_t width;
+    float t_seg, t_persist;
+};
+
+static std::mutex g_choice_mu;
+static std::map<std::vector<std::array<int, 6>>, BatchChoice> g_choices;
+constexpr size_t BATCH_CHOICES_MAX = 1024;  // then they are raced anew
+
+static std::vector<std::array<int, 6>> choice_key(const fft3d_b200_batch *b)
+{
+    std::vector<std::array<int, 6>> key;
+    key.push_back({b->device, b->cls, b->use_graph ? 1 : 0, 0, 0, 0});
+    for (const fft3d_b200_segment &s : b->segs) {
+        int bits = 0;
+        while (bits < 62 && s.batch >> bits > 1) ++bits;
+        key.push_back({s.n0, s.n1, s.n2, s.precision, s.direction, s.batch > 0 ? bits : -1});
+    }
+    return key;
+}
 
 static void batch_free(fft3d_b200_batch *b)
 {
@@ -169,22 +197,22 @@ static cudaError_t batch_enqueue(fft3d_b200_batch *b, cudaStream_t s)
 static cudaError_t segments_enqueue(fft3d_b200_batch *b, cudaStream_t s)
 {
     cudaError_t e = cudaEventRecord(b->fork, s);
-    for (size_t k = 0; k < b->branch.size() && e == cudaSuccess; ++k)
+    for (size_t k = 0; k < b->width && e == cudaSuccess; ++k)
         e = cudaStreamWaitEvent(b->branch[k], b->fork, 0);
     for (size_t i = 0; i < b->plans.size() && e == cudaSuccess; ++i) {
         if (!b->plans[i]) continue;
         const int st = fft3d_b200_execute(b->plans[i], b->segs[i].in, b->segs[i].out,
-                                          b->branch[i % b->branch.size()]);
+                                          b->branch[i % b->width]);
         if (st != FFT3D_B200_OK) e = cudaErrorLaunchFailure;
     }
-    for (size_t k = 0; k < b->branch.size() && e == cudaSuccess; ++k) {
+    for (size_t k = 0; k < b->width && e == cudaSuccess; ++k) {
         e = cudaEventRecord(b->join[k], b->branch[k]);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(s, b->join[k], 0);
     }
     return e;
 }
 
-// Mean time of `reps` runs of a strategy on s (after two warm-up runs): its
+// Mean time of `reps` runs of a strategy on s (after a warm-up run): its
 // graph when the batch replays graphs, its direct launches otherwise.
 static float strategy_time_ms(fft3d_b200_batch *b, bool seg, cudaStream_t s, int reps)
 {
@@ -200,7 +228,7 @@ static float strategy_time_ms(fft3d_b200_batch *b, bool seg, cudaStream_t s, int
         return 1e30f;
     }
     float best = 1e30f;
-    for (int w = 0; w < 2; ++w) run();
+    run();
     for (int r = 0; r < 3; ++r) {
         cudaEventRecord(a, s);
         for (int i = 0; i < reps; ++i) run();
@@ -400,20 +428,78 @@ extern "C" int fft3d_b200_batch_create(const fft3d_b200_segment *segs, int nseg,
                 return fail(FFT3D_B200_ERR_CUDA);
         if (cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) != cudaSuccess)
             return fail(FFT3D_B200_ERR_CUDA);
-        if (b->use_graph) {
-            if (cudaStreamBeginCapture(b->cap, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
-                return fail(FFT3D_B200_ERR_CUDA);
-            cudaError_t le = segments_enqueue(b, b->cap);
-            cudaError_t ee = cudaStreamEndCapture(b->cap, &b->sgraph);
-            if (le != cudaSuccess || ee != cudaSuccess) return fail(FFT3D_B200_ERR_CUDA);
-            if (cudaGraphInstantiate(&b->sexec, b->sgraph, 0) != cudaSuccess) return fail(FFT3D_B200_ERR_CUDA);
+        // One branch a segment runs segments too small for the GPU side by side.  Where
+        // they fill it, so many kernels at once delay one another's last waves, and five
+        // or three branches can be faster: those are timed too for segments of 16 MB of
+        // input and output or more on average (347 MB of complex64 in 8 segments: 8
+        // branches 103.5 us, 5 99.5, 3 103.2; 694 MB of complex128: 182, 181 and 170 us;
+        // 5 to 40 MB in all: one branch a segment, 33.2 us against 40.6 with three).
+        double bytes = 0;
+        for (int i = 0; i < nseg; ++i)
+            bytes += 2.0 * (double)segs[i].batch * segs[i].n0 * segs[i].n1 * segs[i].n2 *
+                     element_bytes(segs[i].precision);
+        const bool race = !(flags & FFT3D_B200_BATCH_SEGMENTS) && persistent_ok;
+        std::vector<size_t> widths = {(size_t)nbr};
+        BatchChoice known = {0, -1.f, -1.f};
+        if (race) {
+            std::lock_guard<std::mutex> lk(g_choice_mu);
+            const auto it = g_choices.find(choice_key(b));
+            if (it != g_choices.end()) known = it->second;
+        }
+        if (known.width) {
+            widths = {known.width};
+        } else {
+            for (size_t w : {(size_t)5, (size_t)3})
+                if (race && bytes / nseg >= 16.0 * 1048576 && w < (size_t)nbr) widths.push_back(w);
         }
         b->segments = true;
-        if (!(flags & FFT3D_B200_BATCH_SEGMENTS) && persistent_ok) {
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t exec = nullptr;
+        size_t width = 0;
+        auto give_up = [&]() {
+            if (exec) cudaGraphExecDestroy(exec);
+            if (graph) cudaGraphDestroy(graph);
+            return fail(FFT3D_B200_ERR_CUDA);
+        };
+        for (size_t w : widths) {
+            b->width = w;
+            if (b->use_graph) {
+                if (cudaStreamBeginCapture(b->cap, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
+                    return give_up();
+                cudaError_t le = segments_enqueue(b, b->cap);
+                cudaError_t ee = cudaStreamEndCapture(b->cap, &b->sgraph);
+                if (le != cudaSuccess || ee != cudaSuccess) return give_up();
+                if (cudaGraphInstantiate(&b->sexec, b->sgraph, 0) != cudaSuccess) return give_up();
+            }
             // the race, on the batch's own buffers
-            t_seg = strategy_time_ms(b, true, b->cap, 5);
-            t_persist = strategy_time_ms(b, false, b->cap, 5);
+            const float t = !race ? 0.f : known.width ? known.t_seg : strategy_time_ms(b, true, b->cap, 2);
+            if (width == 0 || t < t_seg) {
+                std::swap(graph, b->sgraph);
+                std::swap(exec, b->sexec);
+                width = w;
+                t_seg = t;
+            }
+            if (b->sexec) cudaGraphExecDestroy(b->sexec);
+            if (b->sgraph) cudaGraphDestroy(b->sgraph);
+            b->sexec = nullptr;
+            b->sgraph = nullptr;
+        }
+        b->sgraph = graph;
+        b->sexec = exec;
+        b->width = width;
+        if (race) {
+            t_persist = known.width ? known.t_persist : strategy_time_ms(b, false, b->cap, 2);
             b->segments = t_seg < t_persist;
+            if (known.width) {  // a race's launches have the graph on the device already
+                if (b->use_graph && cudaGraphUpload(b->segments ? b->sexec : b->exec, b->cap) != cudaSuccess)
+                    return fail(FFT3D_B200_ERR_CUDA);
+            } else {
+                std::lock_guard<std::mutex> lk(g_choice_mu);
+                if (g_choices.size() >= BATCH_CHOICES_MAX) g_choices.clear();
+                g_choices[choice_key(b)] = {width, t_seg, t_persist};
+            }
+        } else {
+            t_seg = -1.f;
         }
         if (cudaStreamSynchronize(b->cap) != cudaSuccess) return fail(FFT3D_B200_ERR_CUDA);
     }
@@ -421,7 +507,7 @@ extern "C" int fft3d_b200_batch_create(const fft3d_b200_segment *segs, int nseg,
     if (b->segments) {
         snprintf(buf, sizeof buf,
                  "batch: %d segments, one tuned plan per segment on %zu parallel branches, %s",
-                 nseg, b->branch.size(), b->use_graph ? "CUDA graph" : "direct launches");
+                 nseg, b->width, b->use_graph ? "CUDA graph" : "direct launches");
     } else {
         snprintf(buf, sizeof buf, "batch: %d segments, %d items, grid %d x %d threads (%s kernel), %s%s",
                  nseg, b->nitems, b->grid, kernel_class(b->cls).threads,
