@@ -214,6 +214,10 @@ static cudaError_t segments_enqueue(fft3d_b200_batch *b, cudaStream_t s)
 
 // Mean time of `reps` runs of a strategy on s (after a warm-up run): its
 // graph when the batch replays graphs, its direct launches otherwise.
+// Runs a timing.  With two, a race of the 8-segment complex64 mix took 8 branches
+// (110 us in use) in one process of five; with eight, 5 or 3 in all (99.8-101.4 us).
+constexpr int RACE_REPS = 8;
+
 static float strategy_time_ms(fft3d_b200_batch *b, bool seg, cudaStream_t s, int reps)
 {
     auto run = [&]() {
@@ -472,7 +476,7 @@ extern "C" int fft3d_b200_batch_create(const fft3d_b200_segment *segs, int nseg,
                 if (cudaGraphInstantiate(&b->sexec, b->sgraph, 0) != cudaSuccess) return give_up();
             }
             // the race, on the batch's own buffers
-            const float t = !race ? 0.f : known.width ? known.t_seg : strategy_time_ms(b, true, b->cap, 2);
+            const float t = !race ? 0.f : known.width ? known.t_seg : strategy_time_ms(b, true, b->cap, RACE_REPS);
             if (width == 0 || t < t_seg) {
                 std::swap(graph, b->sgraph);
                 std::swap(exec, b->sexec);
@@ -488,7 +492,7 @@ extern "C" int fft3d_b200_batch_create(const fft3d_b200_segment *segs, int nseg,
         b->sexec = exec;
         b->width = width;
         if (race) {
-            t_persist = known.width ? known.t_persist : strategy_time_ms(b, false, b->cap, 2);
+            t_persist = known.width ? known.t_persist : strategy_time_ms(b, false, b->cap, RACE_REPS);
             b->segments = t_seg < t_persist;
             if (known.width) {  // a race's launches have the graph on the device already
                 if (b->use_graph && cudaGraphUpload(b->segments ? b->sexec : b->exec, b->cap) != cudaSuccess)
