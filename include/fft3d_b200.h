@@ -275,11 +275,15 @@ int fft3d_b200_server_submit_many(fft3d_b200_server *server, const fft3d_b200_se
                                   const double *arrival_s, int n, unsigned long long *tickets);
 
 /* Tickets of requests finished since the last poll, in completion order; returns
- * how many were written (<= max). */
+ * how many were written (<= max).  A launch that failed, or in which a bounded
+ * device-side wait ran out, has not written all its outputs: its requests' tickets
+ * never come, and from then on fft3d_b200_server_drain and _get_stats return that
+ * status (FFT3D_B200_ERR_CUDA, FFT3D_B200_ERR_TIMEOUT), and poll too where it has no
+ * ticket to give.  The server goes on serving. */
 int fft3d_b200_server_poll(fft3d_b200_server *server, unsigned long long *tickets, int max);
 
-/* Wait until every submitted request has finished (FFT3D_B200_ERR_TIMEOUT after
- * `timeout_s` seconds). */
+/* Wait until every submitted request has finished or failed (FFT3D_B200_ERR_TIMEOUT
+ * after `timeout_s` seconds). */
 int fft3d_b200_server_drain(fft3d_b200_server *server, double timeout_s);
 
 /* Latency percentiles and throughput of everything finished so far. */
@@ -291,6 +295,11 @@ int fft3d_b200_server_get_stats(fft3d_b200_server *server, fft3d_b200_server_sta
  * so a caller can take percentiles over a steady-state window of the stream. */
 long long fft3d_b200_server_latencies(fft3d_b200_server *server, unsigned long long *tickets,
                                       double *latency_s, long long max);
+
+/* Test hook, no counterpart in the reference: make the server's next launch over a
+ * list of 36^3 volumes skip the first volume's plane items, so that it ends after its
+ * bounded wait (about 2 s) with outputs missing. */
+int fft3d_b200_debug_stall_next_list(fft3d_b200_server *server);
 
 void fft3d_b200_server_destroy(fft3d_b200_server *server);
 

@@ -73,6 +73,10 @@ void register_trip_kernels(std::vector<KernelEntry> &out);     // trip_kernels.c
 // plane items and the row items of one volume in the ticket order (D < R).
 int twopass_ring(const KernelEntry &e, long long grid, int *lag);
 
+// The first row item's ticket in a launch of `e` over `nvol` volumes with up to
+// `grid_limit` CTAs: started there, no plane item of volume 0 is handed out.
+unsigned long long twopass_first_row_ticket(const KernelEntry &e, long long nvol, int grid_limit);
+
 // One volume of a list launch (cube_list_entry): its buffers and direction.
 struct TwoPassVol {
     const void *in;

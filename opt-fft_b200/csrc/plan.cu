@@ -722,14 +722,7 @@ extern "C" int fft3d_b200_debug_stall_next_execute(fft3d_b200_plan *p)
     if (!p) return set_status(FFT3D_B200_ERR_INVALID);
     if (p->kernel->family != FAM_TWOPASS || !p->work[0] || p->desc.batch < 1)
         return set_status(FFT3D_B200_ERR_UNSUPPORTED);
-    const KernelEntry &e = *p->kernel;
-    const long long na = e.n0 / e.vpc, nb = e.n1 / e.vpc;
-    const long long grid = std::max(1LL, std::min((na + nb) * p->desc.batch, (long long)p->grid_limit));
-    int lag = 0;
-    twopass_ring(e, grid, &lag);
-    const long long nvol = p->desc.batch;
-    const unsigned long long first_row = nvol <= lag ? (unsigned long long)(na * nvol)
-                                                     : (unsigned long long)(na * lag + na);
+    const unsigned long long first_row = twopass_first_row_ticket(*p->kernel, p->desc.batch, p->grid_limit);
     int prev = -1;
     cudaGetDevice(&prev);
     if (prev != p->device) cudaSetDevice(p->device);

@@ -9,7 +9,9 @@
 // while batches are running are admitted as soon as a stream slot and budget are
 // free, so their work overlaps the running batches on the device.  Completion is
 // detected with one event per launch; latency is completion minus submission,
-// on the host clock, and p50 / p99 are reported with throughput.
+// on the host clock, and p50 / p99 are reported with throughput.  A launch whose
+// kernels record a bounded wait that ran out has not written all its outputs: its
+// requests end, but are not reported as completed.
 //
 // Each stream slot owns device-resident descriptor buffers, a ticket, and the
 // per-CTA scratch of the two-phase 36^3 route, allocated once at creation; the
@@ -75,7 +77,12 @@ struct ServeSlot {
     unsigned int *d_ticket = nullptr;
     unsigned char *d_solo = nullptr;
     unsigned char *d_scratch = nullptr;
-    int *d_err = nullptr;
+    // The slot's error word, in mapped host memory: kernels write it only when a bounded
+    // wait runs out, and the host reads it when the slot's event has passed, without a
+    // copy in the stream of every launch.
+    volatile int *h_err = nullptr;
+    int *d_err = nullptr;          // its device address
+    int status = FFT3D_B200_OK;    // of the launch calls
     BatchItem *h_items = nullptr;  // pinned staging
     BatchSeg *h_segs = nullptr;
     void *d_work = nullptr;        // workspace of scratch-ring kernels, grown on demand
@@ -106,6 +113,7 @@ struct fft3d_b200_server {
     std::deque<unsigned long long> completed;
     unsigned long long next_ticket = 1;
     unsigned long long submitted = 0, finished = 0;
+    std::atomic<bool> stall_list{false};  // fft3d_b200_debug_stall_next_list
     std::atomic<bool> stop{false};
     std::thread thr;
     int status = FFT3D_B200_OK;
@@ -190,16 +198,22 @@ static_assert(sizeof(TwoPassVol) <= sizeof(BatchItem) && alignof(TwoPassVol) <= 
 static int launch_cubes(fft3d_b200_server *s, ServeSlot &slot, int precision, long long first, long long n)
 {
     const KernelEntry &e = cube_list_entry(precision);
+    const int grid = s->cube_grid[precision == FFT3D_B200_C128 ? 0 : 1];
+    if (s->stall_list.exchange(false)) {
+        const unsigned long long t = twopass_first_row_ticket(e, n, grid);
+        if (cudaMemcpyAsync(slot.d_scratch, &t, sizeof t, cudaMemcpyHostToDevice, slot.stream) != cudaSuccess)
+            return FFT3D_B200_ERR_CUDA;
+    }
     if (cudaMemcpyAsync(slot.d_items + first, slot.h_items + first, (size_t)n * sizeof(TwoPassVol),
                         cudaMemcpyHostToDevice, slot.stream) != cudaSuccess ||
-        launch_entry(e, slot.d_items + first, nullptr, n, 1.0 / (36.0 * 36.0 * 36.0), slot.stream,
-                     s->cube_grid[precision == FFT3D_B200_C128 ? 0 : 1], slot.d_err, slot.d_scratch) != cudaSuccess)
+        launch_entry(e, slot.d_items + first, nullptr, n, 1.0 / (36.0 * 36.0 * 36.0), slot.stream, grid,
+                     slot.d_err, slot.d_scratch) != cudaSuccess)
         return FFT3D_B200_ERR_CUDA;
     return FFT3D_B200_OK;
 }
 
 // Launch every request of `slot` as one persistent batch (or, in plain mode,
-// one launch per request) and record the slot's completion event.
+// one launch per request).
 static int launch_slot(fft3d_b200_server *s, ServeSlot &slot)
 {
     cudaStream_t st = slot.stream;
@@ -305,7 +319,6 @@ static int launch_slot(fft3d_b200_server *s, ServeSlot &slot)
                                       (size_t)batch_kernel_smem(), st) != cudaSuccess)
             return FFT3D_B200_ERR_CUDA;
     }
-    if (cudaEventRecord(slot.done, st) != cudaSuccess) return FFT3D_B200_ERR_CUDA;
     return FFT3D_B200_OK;
 }
 
@@ -345,13 +358,19 @@ static void server_loop(fft3d_b200_server *s)
             const cudaError_t q = cudaEventQuery(slot.done);
             if (q == cudaErrorNotReady) continue;
             const double t = now_s();
-            if (q != cudaSuccess) s->status = FFT3D_B200_ERR_CUDA;
+            int st = slot.status;
+            if (q != cudaSuccess) st = FFT3D_B200_ERR_CUDA;
+            else if (st == FFT3D_B200_OK && *slot.h_err != 0) st = FFT3D_B200_ERR_TIMEOUT;
+            *slot.h_err = 0;
+            slot.status = FFT3D_B200_OK;
+            if (st != FFT3D_B200_OK) s->status = st;
             for (const ServeReq &r : slot.reqs) {
+                ++s->finished;
+                if (st != FFT3D_B200_OK) continue;  // outputs missing: not reported as completed
                 s->lat.push_back(t - r.t_submit);
                 s->lat_ticket.push_back(r.ticket);
                 s->completed.push_back(r.ticket);
                 s->volumes += r.seg.batch;
-                ++s->finished;
             }
             s->t_last = t;
             s->used -= slot.bytes;
@@ -395,11 +414,10 @@ static void server_loop(fft3d_b200_server *s)
         // the slots are this thread's own until they are retired above
         lk.unlock();
         for (ServeSlot *slot : to_launch) {
-            const int st = launch_slot(s, *slot);
-            if (st) {
-                std::lock_guard<std::mutex> g(s->mu);
-                s->status = st;
-            }
+            slot->status = launch_slot(s, *slot);
+            // recorded after a failed launch too: what was launched before it still runs
+            if (cudaEventRecord(slot->done, slot->stream) != cudaSuccess && slot->status == FFT3D_B200_OK)
+                slot->status = FFT3D_B200_ERR_CUDA;
         }
     }
 }
@@ -418,7 +436,7 @@ static void server_free(fft3d_b200_server *s)
         cudaFree(slot.d_ticket);
         cudaFree(slot.d_solo);
         cudaFree(slot.d_scratch);
-        cudaFree(slot.d_err);
+        if (slot.h_err) cudaFreeHost(const_cast<int *>(slot.h_err));
         if (slot.h_items) cudaFreeHost(slot.h_items);
         if (slot.h_segs) cudaFreeHost(slot.h_segs);
     }
@@ -474,9 +492,10 @@ extern "C" int fft3d_b200_server_create(size_t hbm_budget_bytes, int max_infligh
     for (ServeSlot &slot : s->slots) {
         if (cudaStreamCreateWithFlags(&slot.stream, cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreateWithFlags(&slot.done, cudaEventDisableTiming) != cudaSuccess ||
-            cudaMalloc(&slot.d_err, sizeof(int)) != cudaSuccess ||
-            cudaMemset(slot.d_err, 0, sizeof(int)) != cudaSuccess)
+            cudaHostAlloc((void **)&slot.h_err, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
+            cudaHostGetDevicePointer((void **)&slot.d_err, const_cast<int *>(slot.h_err), 0) != cudaSuccess)
             return fail(FFT3D_B200_ERR_NOMEM);
+        *slot.h_err = 0;
         if (!(flags & FFT3D_B200_SERVE_PLAIN)) {
             if (cudaMalloc(&slot.d_items, sizeof(BatchItem) * SERVE_MAX_ITEMS) != cudaSuccess ||
                 cudaMalloc(&slot.d_segs, sizeof(BatchSeg) * SERVE_MAX_SEGS) != cudaSuccess ||
@@ -577,7 +596,17 @@ extern "C" int fft3d_b200_server_poll(fft3d_b200_server *s, unsigned long long *
         tickets[n++] = s->completed.front();
         s->completed.pop_front();
     }
-    return n;
+    return n == 0 && max > 0 ? s->status : n;
+}
+
+// Test hook: the next list launch starts at its first row item's ticket, as
+// fft3d_b200_debug_stall_next_execute makes a plan do.
+extern "C" int fft3d_b200_debug_stall_next_list(fft3d_b200_server *s)
+{
+    if (!s) return FFT3D_B200_ERR_INVALID;
+    if (s->flags & FFT3D_B200_SERVE_PLAIN) return FFT3D_B200_ERR_UNSUPPORTED;
+    s->stall_list.store(true);
+    return FFT3D_B200_OK;
 }
 
 extern "C" int fft3d_b200_server_drain(fft3d_b200_server *s, double timeout_s)

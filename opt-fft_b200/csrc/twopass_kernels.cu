@@ -829,6 +829,14 @@ int twopass_ring(const KernelEntry &e, long long grid, int *lag)
     return r;
 }
 
+unsigned long long twopass_first_row_ticket(const KernelEntry &e, long long nvol, int grid_limit)
+{
+    const long long na = e.n0 / e.vpc, nb = e.n1 / e.vpc;
+    int lag = 0;
+    twopass_ring(e, std::max(1LL, std::min((na + nb) * nvol, (long long)grid_limit)), &lag);
+    return (unsigned long long)(nvol <= lag ? na * nvol : na * lag + na);
+}
+
 size_t entry_workspace_bytes(const KernelEntry &e, int grid_limit)
 {
     if (e.family != FAM_TWOPASS) return 0;

@@ -115,7 +115,7 @@ EXPORTS = {
                      "fft3d_b200_server_submit_many",
                      "fft3d_b200_server_poll", "fft3d_b200_server_drain",
                      "fft3d_b200_server_get_stats", "fft3d_b200_server_latencies",
-                     "fft3d_b200_server_destroy"],
+                     "fft3d_b200_debug_stall_next_list", "fft3d_b200_server_destroy"],
 }
 
 
@@ -191,6 +191,7 @@ def _load():
         "fft3d_b200_server_get_stats": ([vp, ctypes.POINTER(ServerStats)], i),
         "fft3d_b200_server_latencies": ([vp, ctypes.POINTER(ctypes.c_ulonglong),
                                          ctypes.POINTER(ctypes.c_double), ll], ll),
+        "fft3d_b200_debug_stall_next_list": ([vp], i),
         "fft3d_b200_server_destroy": ([vp], None),
     }
     for name, (args, res) in sig.items():
