@@ -395,6 +395,7 @@ extern "C" int fft3d_b200_batch_create(const fft3d_b200_segment *segs, int nseg,
     }
     // The per-segment strategy: built unless the persistent kernel is pinned
     // (or timing is off), then timed against the persistent launch.
+    bool remembered = false;  // the times are another batch's (BatchChoice)
     const bool want_seg = !persistent_ok || (flags & FFT3D_B200_BATCH_SEGMENTS) ||
                           !(flags & (FFT3D_B200_BATCH_PERSISTENT | FFT3D_B200_FLAG_NO_TUNE));
     float t_persist = -1.f, t_seg = -1.f;
@@ -451,6 +452,7 @@ extern "C" int fft3d_b200_batch_create(const fft3d_b200_segment *segs, int nseg,
             if (it != g_choices.end()) known = it->second;
         }
         if (known.width) {
+            remembered = true;
             widths = {known.width};
         } else {
             for (size_t w : {(size_t)5, (size_t)3})
@@ -520,8 +522,8 @@ extern "C" int fft3d_b200_batch_create(const fft3d_b200_segment *segs, int nseg,
     }
     b->describe = buf;
     if (t_seg >= 0.f) {
-        snprintf(buf, sizeof buf, " (timed: per-segment %.1f us, persistent %.1f us)", t_seg * 1e3f,
-                 t_persist * 1e3f);
+        snprintf(buf, sizeof buf, " (timed: per-segment %.1f us, persistent %.1f us%s)", t_seg * 1e3f,
+                 t_persist * 1e3f, remembered ? "; by an earlier batch" : "");
         b->describe += buf;
     }
     if (prev >= 0 && prev != device) cudaSetDevice(prev);
