@@ -12,7 +12,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <array>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -22,6 +21,7 @@
 #include <vector>
 
 #include "../../include/fft3d_b200.h"
+#include "batch_choice.h"
 #include "batch_kinds.h"
 #include "internal.h"
 #include "volume.cuh"
@@ -129,27 +129,20 @@ struct fft3d_b200_batch {
 };
 
 // What a race between the strategies found, kept per process for batches of the same
-// segments (up to the size class of their volume counts) as the autotuner keeps its
-// choices: a program that makes a batch for each set of buffers races once.
+// segments (batch_choice.h): a program that makes a batch for each set of buffers
+// races once.
 struct BatchChoice {
     size_t width;
     float t_seg, t_persist;
 };
 
 static std::mutex g_choice_mu;
-static std::map<std::vector<std::array<int, 6>>, BatchChoice> g_choices;
+static std::map<BatchChoiceKey, BatchChoice> g_choices;
 constexpr size_t BATCH_CHOICES_MAX = 1024;  // then they are raced anew
 
-static std::vector<std::array<int, 6>> choice_key(const fft3d_b200_batch *b)
+static BatchChoiceKey choice_key(const fft3d_b200_batch *b)
 {
-    std::vector<std::array<int, 6>> key;
-    key.push_back({b->device, b->cls, b->use_graph ? 1 : 0, 0, 0, 0});
-    for (const fft3d_b200_segment &s : b->segs) {
-        int bits = 0;
-        while (bits < 62 && s.batch >> bits > 1) ++bits;
-        key.push_back({s.n0, s.n1, s.n2, s.precision, s.direction, s.batch > 0 ? bits : -1});
-    }
-    return key;
+    return batch_choice_key(b->device, b->cls, b->use_graph, b->segs.data(), b->segs.size());
 }
 
 static void batch_free(fft3d_b200_batch *b)

@@ -13,6 +13,7 @@
 #include <array>
 #include <vector>
 
+#include "batch_choice.h"
 #include "staged.cuh"
 #include "mgpu.cuh"
 #include "splitline.cuh"
@@ -837,6 +838,12 @@ static void emulate_tpass(cx<double> *data, long long vol_elems, long long batch
             dft<TL, SGN, double>(v);
             for (int t = 0; t < TL; ++t) col[t * vol_elems] = SGN > 0 ? cscale(v[t], scale) : v[t];
         }
+}
+
+// Whether two batches' segments may share a race's result (batch_choice.h).
+extern "C" int hostcheck_same_choice(const fft3d_b200_segment *a, int na, const fft3d_b200_segment *b, int nb)
+{
+    return batch_choice_key(0, 1, true, a, (size_t)na) == batch_choice_key(0, 1, true, b, (size_t)nb);
 }
 
 extern "C" int hostcheck_tpass(int tl, int sign, void *data, long long vol_elems, long long batch)
