@@ -146,10 +146,12 @@ const char *fft3d_b200_status_string(int status);
 /* Write the choices made or imported so far; entries written, or an error code. */
 int fft3d_b200_wisdom_export(const char *path);
 
-/* Merge a wisdom file into this process's choices; entries taken, or an error code. */
+/* Merge a wisdom file into this process's choices; entries taken, or an error code.
+ * Batches created afterwards time their strategies again, with the imported kernels. */
 int fft3d_b200_wisdom_import(const char *path);
 
-/* Drop every remembered choice (plans created afterwards time their candidates again). */
+/* Drop every remembered choice (plans created afterwards time their candidates again,
+ * batches their strategies). */
 void fft3d_b200_wisdom_forget(void);
 
 /* ---------------------------------------------------------------- 4D lattices (L^3 x T)

@@ -138,7 +138,16 @@ struct BatchChoice {
 
 static std::mutex g_choice_mu;
 static std::map<BatchChoiceKey, BatchChoice> g_choices;
+static unsigned long long g_choices_forgotten = 0;  // times
 constexpr size_t BATCH_CHOICES_MAX = 1024;  // then they are raced anew
+
+// The choices were raced with the plans that the autotuner's choices make.
+void fft3d::forget_batch_choices()
+{
+    std::lock_guard<std::mutex> lk(g_choice_mu);
+    g_choices.clear();
+    ++g_choices_forgotten;
+}
 
 static BatchChoiceKey choice_key(const fft3d_b200_batch *b)
 {
@@ -389,6 +398,11 @@ extern "C" int fft3d_b200_batch_create(const fft3d_b200_segment *segs, int nseg,
     // The per-segment strategy: built unless the persistent kernel is pinned
     // (or timing is off), then timed against the persistent launch.
     bool remembered = false;  // the times are another batch's (BatchChoice)
+    unsigned long long forgotten = 0;
+    {
+        std::lock_guard<std::mutex> lk(g_choice_mu);
+        forgotten = g_choices_forgotten;
+    }
     const bool want_seg = !persistent_ok || (flags & FFT3D_B200_BATCH_SEGMENTS) ||
                           !(flags & (FFT3D_B200_BATCH_PERSISTENT | FFT3D_B200_FLAG_NO_TUNE));
     float t_persist = -1.f, t_seg = -1.f;
@@ -495,7 +509,8 @@ extern "C" int fft3d_b200_batch_create(const fft3d_b200_segment *segs, int nseg,
             } else {
                 std::lock_guard<std::mutex> lk(g_choice_mu);
                 if (g_choices.size() >= BATCH_CHOICES_MAX) g_choices.clear();
-                g_choices[choice_key(b)] = {width, t_seg, t_persist};
+                // raced with plans made before the last forget: not kept
+                if (forgotten == g_choices_forgotten) g_choices[choice_key(b)] = {width, t_seg, t_persist};
             }
         } else {
             t_seg = -1.f;

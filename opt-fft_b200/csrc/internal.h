@@ -113,6 +113,9 @@ int entry_occupancy(const KernelEntry &e, int device);
 
 int element_bytes(int precision);
 
+// Drop every batch's remembered choice between the launch strategies (batch.cu).
+void forget_batch_choices();
+
 // The autotuner's choice for a geometry at a batch size (memoised per batch
 // bucket like plan creation); nullptr if the geometry has no kernel.  Without
 // `workspace_ok` it chooses among the kernels that need no workspace (a caller

@@ -537,6 +537,7 @@ extern "C" int fft3d_b200_wisdom_import(const char *path)
     if (!path) return fft3d::set_status(FFT3D_B200_ERR_INVALID);
     std::lock_guard<std::mutex> lk(fft3d::g_tune_mu);
     const int n = fft3d::wisdom_read(path);
+    if (n > 0) fft3d::forget_batch_choices();
     fft3d::set_status(n < 0 ? n : FFT3D_B200_OK);
     return n;
 }
@@ -546,6 +547,7 @@ extern "C" void fft3d_b200_wisdom_forget(void)
     std::lock_guard<std::mutex> lk(fft3d::g_tune_mu);
     fft3d::g_tuned.clear();
     fft3d::g_wisdom_foreign.clear();
+    fft3d::forget_batch_choices();
 }
 
 // Allocate workspace `i` of a plan whose kernel needs one; its control block

@@ -42,3 +42,27 @@ def test_second_batch_of_the_same_segments(bytes_in, flags, nseg):
     # the second raced nothing: the first's choice, and its times as an earlier batch's
     assert notes[1] == notes[0].replace(" us)", " us; by an earlier batch)")
     assert "by an earlier batch" in notes[1]
+
+
+def test_forgotten_with_the_plans_choices(tmp_path):
+    """A batch's choice was timed with the kernels that the plans' choices name."""
+    a = torch.zeros((500, 12, 12, 12), dtype=torch.complex128, device="cuda")
+    b = torch.zeros_like(a)
+
+    def remembered():
+        batch = fb.Batch([dict(shape=(12, 12, 12), batch=250, **{"in": a[k:].data_ptr()}, out=b[k:].data_ptr())
+                          for k in (0, 250)])
+        note = batch.describe()
+        batch.close()
+        assert "timed" in note
+        return "by an earlier batch" in note
+
+    fb.wisdom_forget()
+    assert [remembered(), remembered()] == [False, True]
+    fb.wisdom_forget()
+    assert [remembered(), remembered()] == [False, True]
+    fb.wisdom_export(tmp_path / "w.txt")
+    assert remembered()
+    assert fb.wisdom_import(tmp_path / "w.txt") > 0
+    assert [remembered(), remembered()] == [False, True]
+    fb.wisdom_forget()
