@@ -214,36 +214,36 @@ static cudaError_t segments_enqueue(fft3d_b200_batch *b, cudaStream_t s)
     return e;
 }
 
-// Mean time of `reps` runs of a strategy on s (after a warm-up run): its
-// graph when the batch replays graphs, its direct launches otherwise.
 // Runs a timing.  With two, a race of the 8-segment complex64 mix took 8 branches
 // (110 us in use) in one process of five; with eight, 5 or 3 in all (99.8-101.4 us).
 constexpr int RACE_REPS = 8;
 
+// Mean time of `reps` runs of a strategy on s (after a warm-up run): its
+// graph when the batch replays graphs, its direct launches otherwise.
+// RACE_FAILED_MS if a call fails.
 static float strategy_time_ms(fft3d_b200_batch *b, bool seg, cudaStream_t s, int reps)
 {
     auto run = [&]() {
-        if (b->use_graph) cudaGraphLaunch(seg ? b->sexec : b->exec, s);
-        else if (seg) segments_enqueue(b, s);
-        else batch_enqueue(b, s);
+        if (b->use_graph) return cudaGraphLaunch(seg ? b->sexec : b->exec, s) == cudaSuccess;
+        return (seg ? segments_enqueue(b, s) : batch_enqueue(b, s)) == cudaSuccess;
     };
     cudaEvent_t a, z;
-    if (cudaEventCreate(&a) != cudaSuccess) return 1e30f;
+    if (cudaEventCreate(&a) != cudaSuccess) return RACE_FAILED_MS;
     if (cudaEventCreate(&z) != cudaSuccess) {
         cudaEventDestroy(a);
-        return 1e30f;
+        return RACE_FAILED_MS;
     }
-    float best = 1e30f;
-    run();
-    for (int r = 0; r < 3; ++r) {
-        cudaEventRecord(a, s);
-        for (int i = 0; i < reps; ++i) run();
-        cudaEventRecord(z, s);
-        cudaEventSynchronize(z);
+    float best = RACE_FAILED_MS;
+    bool ok = run();
+    for (int r = 0; r < 3 && ok; ++r) {
+        ok = cudaEventRecord(a, s) == cudaSuccess;
+        for (int i = 0; i < reps && ok; ++i) ok = run();
         float ms = 0.f;
-        cudaEventElapsedTime(&ms, a, z);
+        ok = ok && cudaEventRecord(z, s) == cudaSuccess && cudaEventSynchronize(z) == cudaSuccess &&
+             cudaEventElapsedTime(&ms, a, z) == cudaSuccess;
         best = std::min(best, ms / (float)reps);
     }
+    if (!ok) best = RACE_FAILED_MS;
     cudaEventDestroy(a);
     cudaEventDestroy(z);
     cudaGetLastError();
@@ -503,19 +503,19 @@ extern "C" int fft3d_b200_batch_create(const fft3d_b200_segment *segs, int nseg,
         if (race) {
             t_persist = known.width ? known.t_persist : strategy_time_ms(b, false, b->cap, RACE_REPS);
             b->segments = t_seg < t_persist;
-            if (known.width) {  // a race's launches have the graph on the device already
-                if (b->use_graph && cudaGraphUpload(b->segments ? b->sexec : b->exec, b->cap) != cudaSuccess)
-                    return fail(FFT3D_B200_ERR_CUDA);
-            } else {
-                std::lock_guard<std::mutex> lk(g_choice_mu);
-                if (g_choices.size() >= BATCH_CHOICES_MAX) g_choices.clear();
-                // raced with plans made before the last forget: not kept
-                if (forgotten == g_choices_forgotten) g_choices[choice_key(b)] = {width, t_seg, t_persist};
-            }
-        } else {
-            t_seg = -1.f;
+            // a race's launches have the graph on the device already
+            if (known.width && b->use_graph &&
+                cudaGraphUpload(b->segments ? b->sexec : b->exec, b->cap) != cudaSuccess)
+                return fail(FFT3D_B200_ERR_CUDA);
         }
         if (cudaStreamSynchronize(b->cap) != cudaSuccess) return fail(FFT3D_B200_ERR_CUDA);
+        if (race && !known.width && race_measured(t_seg, t_persist)) {
+            std::lock_guard<std::mutex> lk(g_choice_mu);
+            if (g_choices.size() >= BATCH_CHOICES_MAX) g_choices.clear();
+            // raced with plans made before the last forget: not kept
+            if (forgotten == g_choices_forgotten) g_choices[choice_key(b)] = {width, t_seg, t_persist};
+        }
+        if (!race) t_seg = -1.f;
     }
     char buf[400];
     if (b->segments) {

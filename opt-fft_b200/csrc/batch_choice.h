@@ -30,4 +30,13 @@ inline BatchChoiceKey batch_choice_key(int device, int cls, bool use_graph, cons
     return key;
 }
 
+// A timing that failed.
+constexpr float RACE_FAILED_MS = 1e30f;
+
+// Whether a race's times may be kept for other batches: both were measured.
+inline bool race_measured(float t_seg, float t_persist)
+{
+    return t_seg > 0.f && t_seg < RACE_FAILED_MS && t_persist > 0.f && t_persist < RACE_FAILED_MS;
+}
+
 }  // namespace fft3d

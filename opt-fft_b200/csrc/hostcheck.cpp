@@ -846,6 +846,11 @@ extern "C" int hostcheck_same_choice(const fft3d_b200_segment *a, int na, const 
     return batch_choice_key(0, 1, true, a, (size_t)na) == batch_choice_key(0, 1, true, b, (size_t)nb);
 }
 
+extern "C" int hostcheck_race_measured(float t_seg, float t_persist)
+{
+    return race_measured(t_seg, t_persist);
+}
+
 extern "C" int hostcheck_tpass(int tl, int sign, void *data, long long vol_elems, long long batch)
 {
     ensure_host_tables();

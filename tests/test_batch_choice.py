@@ -47,3 +47,11 @@ def test_other_buffers_share(same):
 def test_others_race_for_themselves(same, a, b):
     assert not same(a, b)
     assert same(a, list(a)) and same(b, list(b))
+
+
+@pytest.mark.parametrize("t_seg,t_persist,kept", [(0.1, 0.2, True), (0.0, 0.2, False), (0.1, 0.0, False), (1e30, 0.2, False),
+                                                  (0.1, 1e30, False), (float("nan"), 0.2, False), (-1.0, 0.2, False)])
+def test_only_measured_times_are_kept(hostcheck, t_seg, t_persist, kept):
+    f = hostcheck.hostcheck_race_measured
+    f.argtypes = [ctypes.c_float, ctypes.c_float]
+    assert bool(f(t_seg, t_persist)) == kept
