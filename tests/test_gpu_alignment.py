@@ -33,3 +33,30 @@ def test_complex64_off_16_bytes(shape, n, offset_in, offset_out):
         err = oracle.rel_error_per_volume(b[pick].cpu().numpy().astype(np.complex128), want).max()
         assert err < C64_TOL, (v, err)
         plan.close()
+
+
+def microseconds(plan, a, b):
+    best = float("inf")
+    for _ in range(4):
+        t = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        t[0].record()
+        for _ in range(10):
+            plan.execute(a.data_ptr(), b.data_ptr())
+        t[1].record()
+        torch.cuda.synchronize()
+        best = min(best, t[0].elapsed_time(t[1]) * 100)
+    return best
+
+
+# a plan is tuned on aligned buffers and takes any: (shape, volumes, what is slowest allowed against VOLUME)
+SLOWEST = [((30, 30, 30), 300, 1.25)]  # 0.98 measured; 1.7 when one thread copied a chunk of rows
+
+
+@pytest.mark.parametrize("shape,n,most", SLOWEST, ids=[str(c[0]) for c in SLOWEST])
+def test_plans_off_16_bytes_keep_their_speed(shape, n, most):
+    raw = [torch.zeros(8 * n * int(np.prod(shape)) + 16, dtype=torch.uint8, device="cuda")[8:] for _ in range(2)]
+    names = fb.variants(shape, fb.C64)
+    plans = [fb.Plan(shape, n, fb.FORWARD, fb.C64), fb.Plan(shape, n, fb.FORWARD, fb.C64, variant=next(
+        v for v in names if v.startswith("volume")))]
+    tuned, volume = [microseconds(p, *raw) for p in plans]
+    assert tuned < most * volume, (plans[0].describe(), tuned, volume)
