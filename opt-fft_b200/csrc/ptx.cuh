@@ -93,10 +93,15 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar)
 }
 
 // Arrive on the barrier once this thread's cp.async copies so far have completed;
-// the barrier's count has this arrival.
+// the barrier's count has this arrival (noinc), or is raised by it at once (inc).
 __device__ __forceinline__ void cp_async_mbar_arrive_noinc(uint64_t *bar)
 {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+__device__ __forceinline__ void cp_async_mbar_arrive_inc(uint64_t *bar)
+{
+    asm volatile("cp.async.mbarrier.arrive.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)

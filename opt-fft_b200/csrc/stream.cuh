@@ -19,7 +19,12 @@
 //   BULK   (natural layout, odd n2): thread 0 issues one cp.async.bulk (TMA)
 //          per item -- the group is one contiguous byte range -- completing on
 //          the stage's mbarrier.  Items that are not 16-byte aligned in address
-//          or size (complex64 tails of odd volumes) are copied by the threads.
+//          or size (complex64: odd volumes, buffers off 16 bytes) are copied by the
+//          threads' cp.async, which complete on the same mbarrier, and a BST item
+//          whose output is off 16 bytes is stored by its x lines.  48 MB with both
+//          buffers 8 bytes off: 15^3 31.7 us (44.4 when the threads waited for their
+//          copies and copied the outputs out of the stage), 9^3 28.2 (34.0), 3x5x7
+//          31.7 (38.4), 5^3 29.3 (32.6); aligned 23.2, 21.1, 24.9 and 22.3.
 //   ASYNC  (padded or XOR-swizzled layouts): every thread issues cp.async copies
 //          of its elements straight into their layout slots.
 // Every mbarrier wait is bounded (ptx.cuh); a timeout records an error code in
@@ -41,14 +46,6 @@ struct StreamLayout {
     static constexpr int STAGE_BYTES = ((VPC * G::PV * G::EB) + 127) / 128 * 128;
     static constexpr int SMEM_BYTES = NSTAGE * STAGE_BYTES + 8 * NSTAGE;
 };
-
-// Threads copy element by element (synchronous), used for unaligned BULK items.
-template <class G>
-__device__ __forceinline__ void load_lsu(cx<typename G::T> *stage, const cx<typename G::T> *gin,
-                                         int nel, int tid, int nt)
-{
-    for (int g = tid; g < nel; g += nt) stage_in<G>(stage, gin, g);
-}
 
 template <class G, int NT>
 __device__ __forceinline__ void load_async(cx<typename G::T> *stage, const cx<typename G::T> *gin,
@@ -105,7 +102,7 @@ __global__ void __launch_bounds__(NT, MINB)
     __syncthreads();
 
     // Issue the load of `item` into stage s.  For BULK, returns with the copy in
-    // flight (or, for an unaligned item, done by the threads and arrived).
+    // flight: one bulk copy, or the threads' element copies.
     // Both directions walk their items in order.  Starting an inverse on the
     // items a preceding forward wrote last (still partly in L2) -- walking them
     // from last to first, or from the last 32 MB of the batch and wrapping --
@@ -120,16 +117,18 @@ __global__ void __launch_bounds__(NT, MINB)
         const int nel = nv * G::V;
         if constexpr (LOADER == LOADER_BULK) {
             const uint32_t bytes = (uint32_t)nel * (uint32_t)G::EB;
-            const bool aligned = ((((uintptr_t)gin) | bytes) & 15u) == 0;
-            if (aligned) {
-                if (tid == 0) {  // read once: keep L2 for the output
-                    mbar_arrive_expect_tx(&bar[s], bytes);
-                    bulk_g2s_hint(stage(s), gin, bytes, &bar[s], pol_first);
+            if constexpr (G::EB == 8) {
+                if ((((uintptr_t)gin) | bytes) & 15u) {
+                    load_async<G, NT>(stage(s), gin, nel, tid);
+                    cp_async_mbar_arrive_inc(&bar[s]);
+                    __syncthreads();  // every thread has raised the count
+                    if (tid == 0) mbar_arrive(&bar[s]);
+                    return;
                 }
-            } else {
-                load_lsu<G>(stage(s), gin, nel, tid, NT);
-                __syncthreads();
-                if (tid == 0) mbar_arrive(&bar[s]);
+            }
+            if (tid == 0) {  // read once: keep L2 for the output
+                mbar_arrive_expect_tx(&bar[s], bytes);
+                bulk_g2s_hint(stage(s), gin, bytes, &bar[s], pol_first);
             }
         } else {
             load_async<G, NT>(stage(s), gin, nel, tid);
@@ -175,6 +174,14 @@ __global__ void __launch_bounds__(NT, MINB)
         }
         cx<T> *gout = out + v0 * G::V;
         if constexpr (BST) {
+            const uint32_t bytes = (uint32_t)(nv * G::V) * (uint32_t)G::EB;
+            if constexpr (G::EB == 8) {
+                if ((((uintptr_t)gout) | bytes) & 15u) {  // no bulk store: as without BST
+                    for (int l = tid; l < nv * G::N1 * G::N2; l += NT) pass_x_out<G, S, ALG, true>(sm, l, gout, scale);
+                    fence_proxy_async_smem();
+                    continue;  // the stage is refilled after the next item's barriers
+                }
+            }
             // x pass in place, then one bulk store of the group (plain L2 policy:
             // a following transform of this output finds its last part in L2)
             if constexpr (G::POL == 0) {
@@ -188,15 +195,9 @@ __global__ void __launch_bounds__(NT, MINB)
             }
             fence_proxy_async_smem();
             __syncthreads();
-            const uint32_t bytes = (uint32_t)(nv * G::V) * (uint32_t)G::EB;
-            if (((((uintptr_t)gout) | bytes) & 15u) == 0) {
-                if (tid == 0) {
-                    bulk_s2g(gout, sm, bytes);
-                    bulk_commit();
-                }
-            } else {
-                for (int g = tid; g < nv * G::V; g += NT) gout[g] = sm[g];
-                fence_proxy_async_smem();
+            if (tid == 0) {
+                bulk_s2g(gout, sm, bytes);
+                bulk_commit();
             }
         } else {
             // plain stores: a following transform of this output finds its last part in L2
