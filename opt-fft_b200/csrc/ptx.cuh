@@ -143,6 +143,21 @@ __device__ __forceinline__ void named_barrier_sync(int id, int threads)
     asm volatile("barrier.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
+// The same barrier; true when any of the threads passes `stop`.
+__device__ __forceinline__ bool named_barrier_any(int id, int threads, bool stop)
+{
+    uint32_t any;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %3, 0;\n\t"
+        "barrier.red.or.pred q, %1, %2, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(any)
+        : "r"(id), "r"(threads), "r"((uint32_t)stop)
+        : "memory");
+    return any != 0;
+}
+
 // Order this thread's generic-proxy shared-memory accesses before later
 // async-proxy (TMA) accesses of the same memory.
 __device__ __forceinline__ void fence_proxy_async_smem()

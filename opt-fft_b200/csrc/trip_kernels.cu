@@ -118,12 +118,16 @@ __global__ void __launch_bounds__(NT + 32, MINB)
         auto st_ring = [&](cx<T> *p, cx<T> v) { st_hint(p, v, pol_last); };
         auto st_out = [&](cx<T> *p, cx<T> v) { store_out(p, v); };
         for (unsigned k = 0;; ++k) {
-            if (!mbar_wait_timed(&s_full[k & 1], (k >> 1) & 1)) {
-                report_error(err, DEV_ERR_QUEUE_TIMEOUT);
+            // The workers leave together, by a vote at an item's first barrier: one whose
+            // wait ran out while another's was still answered must not be missing at
+            // the barriers that follow.
+            const bool posted = mbar_wait_timed(&s_full[k & 1], (k >> 1) & 1);
+            const long long ticket = *(volatile long long *)&s_mail[k & 1];
+            if (!posted || ticket < 0) {
+                if (!posted) report_error(err, DEV_ERR_QUEUE_TIMEOUT);
+                named_barrier_any(1, NT, true);
                 break;
             }
-            const long long ticket = *(volatile long long *)&s_mail[k & 1];
-            if (ticket < 0) break;
             const TwoPassItem it = twopass_decode(ticket, nvol, TG::NA, TG::NB, D);
             cx<T> *sv = ring + it.vol % R * TG::V;
             cx<T> v[TR::A];
@@ -131,7 +135,7 @@ __global__ void __launch_bounds__(NT + 32, MINB)
                 const long long p0 = (long long)it.j * G * TR::PLANE;
                 const cx<T> *src = in + it.vol * TG::V + p0;
                 if (tid < TR::T1) TR::trip1_load(src, tid, v, ld_in);
-                named_barrier_sync(1, NT);  // the item before has left shared memory
+                if (named_barrier_any(1, NT, false)) break;  // the item before has left shared memory
                 if (tid < TR::T1) TR::template trip1_store<S>(sm, tid, v);
                 for (int t = tid + NT; t < TR::T1; t += NT) {
                     TR::trip1_load(src, t, v, ld_in);
@@ -144,7 +148,7 @@ __global__ void __launch_bounds__(NT + 32, MINB)
             } else {
                 const long long r0 = (long long)it.j * G * N;
                 if (tid < TR::R1) TR::row1_load(sv + r0, tid, v, ld_ring);
-                named_barrier_sync(1, NT);
+                if (named_barrier_any(1, NT, false)) break;
                 if (tid < TR::R1) TR::template row1_store<S>(sm, tid, v);
                 for (int t = tid + NT; t < TR::R1; t += NT) {
                     TR::row1_load(sv + r0, t, v, ld_ring);
