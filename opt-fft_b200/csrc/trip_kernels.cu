@@ -42,7 +42,9 @@ __device__ __forceinline__ bool trip_control(TwoPassCtl *ctl, long long nvol, in
         mbar_arrive(&full[posted & 1]);
     };
     for (;;) {
-        if (freed != posted && mbar_try_wait(&done[freed & 1], (freed >> 1) & 1)) {
+        // test_wait: try_wait may suspend the thread for as long as the item takes, and
+        // the next item's counter would be polled only then
+        if (freed != posted && mbar_test_wait(&done[freed & 1], (freed >> 1) & 1)) {
             red_release_gpu_add(publish, 1u);
             publish = publish_next;
             ++freed;
@@ -192,7 +194,7 @@ static void add_trip(std::vector<KernelEntry> &out, const char *name)
 
 // Measured over 96 MB (floor 30 us at 6.65 TB/s), the staged kernel (two 8-point
 // stages a line through shared memory, twopass_kernels.cu) and this one: 64^3 c128
-// 92.7 / 75.1 us.  Movement through the ring alone, without the trips through
+// 92.7 / 74.0 us.  Movement through the ring alone, without the trips through
 // shared memory or any wait, takes 45 us, the trips add 13 us and the arithmetic
 // 6 us.  Two CTAs of 256 workers an SM; three spill (100 us).  The same split as
 // 9 x 4 for 36^3 takes 74-79 us against 70 us for one line a thread (bulkqh), 8 x 3

@@ -814,7 +814,8 @@ int twopass_ring(const KernelEntry &e, long long grid, int *lag)
 {
     // The lag covers up to twice the tickets the grid holds at once: kernels
     // that take their next ticket ahead (k_twopass_regs, k_twopass_staged) hold
-    // two per CTA, and for the others too a lag of two grids' worth measured
+    // two per CTA (k_trip three, but 64^3 complex double's ring is at its 64 MB with
+    // two grids' worth already: the same lag of 7), and for the others too a lag of two grids' worth measured
     // faster on B200 (fewer row items arriving before their planes are done).
     // It is shortened, down to one grid's worth, while the ring would exceed
     // 64 MB, so that the ring stays in half of L2.
