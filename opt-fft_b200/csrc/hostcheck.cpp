@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "batch_choice.h"
+#include "serve_rule.h"
 #include "staged.cuh"
 #include "mgpu.cuh"
 #include "splitline.cuh"
@@ -849,6 +850,15 @@ extern "C" int hostcheck_same_choice(const fft3d_b200_segment *a, int na, const 
 extern "C" int hostcheck_race_measured(float t_seg, float t_persist)
 {
     return race_measured(t_seg, t_persist);
+}
+
+// serve_rule.h: bit k set when precision k's cubes take a list launch.
+extern "C" int hostcheck_cubes_by_list(int sms, long long n128, long long n64, double other_bytes)
+{
+    const long long n[2] = {n128, n64};
+    bool listed[2] = {false, false};
+    cubes_by_list(sms, n, other_bytes, listed);
+    return (listed[0] ? 1 : 0) + (listed[1] ? 2 : 0);
 }
 
 extern "C" int hostcheck_tpass(int tl, int sign, void *data, long long vol_elems, long long batch)

@@ -20,7 +20,7 @@
 // 36^3 volumes, beyond one SM, take one SM about 100 us each in the persistent
 // kernel (complex double).  Where that is not hidden behind the rest of the batch,
 // the batch's cubes run before it in one TWOPASS launch over all requests' volumes
-// (cubes_by_list).
+// of a precision (serve_rule.h).
 //
 // A request whose extent is not one of the persistent kernel's kinds (any
 // other compiled extent) is launched on its own with its tuned kernel, on the
@@ -46,6 +46,7 @@
 #include "../../include/fft3d_b200.h"
 #include "batch_kinds.h"
 #include "internal.h"
+#include "serve_rule.h"
 
 namespace fft3d {
 
@@ -102,6 +103,7 @@ struct fft3d_b200_server {
     size_t budget = 0;
     size_t used = 0;
     size_t peak_used = 0;
+    int sms = 0;
     int grid = 0;
     long long scratch_per_cta = 0;
     int cube_grid[2] = {0, 0};  // CTAs of a list launch, by precision
@@ -170,22 +172,6 @@ static int launch_request(fft3d_b200_server *s, ServeSlot &slot, const ServeReq 
     return FFT3D_B200_OK;
 }
 
-// Whether the 36^3 volumes of a batch, n of one precision, are faster in a list
-// launch of their own than as items of the persistent kernel beside `other_bytes`
-// of other volumes.  Measured on B200, complex double / float: the list launch takes
-// 12 us + 0.48 / 0.26 us a volume; as an item, a volume holds one SM for 98 / 49 us
-// (0.66 / 0.33 us of the whole GPU), and the batch cannot end before its last one;
-// the other kinds move 2.3 TB/s.
-static bool cubes_by_list(int precision, long long n, double other_bytes)
-{
-    const bool c128 = precision == FFT3D_B200_C128;
-    const double other = other_bytes / 2.3e6;  // us
-    const double list = other + 12.0 + (c128 ? 0.48 : 0.26) * (double)n;
-    const double item = c128 ? 98.0 : 49.0;
-    const double items = std::max(item * (double)((n + 147) / 148), other + item / 148.0 * (double)n);
-    return n > 0 && list < items;
-}
-
 // The volumes of a slot's list launches lie at the end of its item buffers: a cube
 // counts as one item when requests are admitted, and is one or the other.
 static_assert(sizeof(TwoPassVol) <= sizeof(BatchItem) && alignof(TwoPassVol) <= alignof(BatchItem),
@@ -231,13 +217,13 @@ static int launch_slot(fft3d_b200_server *s, ServeSlot &slot)
         double other_bytes = 0;
         for (const ServeReq &r : slot.reqs) {
             if (r.cube) cubes[r.seg.precision == FFT3D_B200_C128 ? 0 : 1] += r.seg.batch;
-            else other_bytes += (double)r.bytes;
+            else if (r.kind >= 0) other_bytes += (double)r.bytes;  // the others were launched above
         }
         bool listed[2];
+        cubes_by_list(s->sms, cubes, other_bytes, listed);
         long long end = SERVE_MAX_ITEMS;  // of the item buffers not taken by volumes
         for (int k = 0; k < 2; ++k) {
             const int precision = k == 0 ? FFT3D_B200_C128 : FFT3D_B200_C64;
-            listed[k] = cubes_by_list(precision, cubes[k], other_bytes);
             if (!listed[k]) continue;
             end -= cubes[k];
             TwoPassVol *vol = reinterpret_cast<TwoPassVol *>(slot.h_items + end);
@@ -477,6 +463,7 @@ extern "C" int fft3d_b200_server_create(size_t hbm_budget_bytes, int max_infligh
                                                       (size_t)batch_kernel_smem()) != cudaSuccess ||
         occ < 1)
         return fail(FFT3D_B200_ERR_UNSUPPORTED);
+    s->sms = sms;
     s->grid = occ * sms;
     s->scratch_per_cta = (long long)36 * 36 * 36 * 16;  // the largest two-phase volume
     // a slot's scratch: the list launches' control block, then the larger of their
