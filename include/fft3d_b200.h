@@ -228,10 +228,14 @@ typedef struct fft3d_b200_chain fft3d_b200_chain;
 int fft3d_b200_chain_create(int n0, int n1, int n2, long long batch, int precision, int kind,
                             const void *d_c, int device, fft3d_b200_chain **out);
 
-/* Run `steps` chain steps from d_x0, leaving the end state in d_out (one launch;
- * each volume stays in one CTA's shared memory for the whole chain). */
+/* Run `steps` chain steps from d_x0, leaving the end state in d_out (one launch; each
+ * volume stays in the shared memory of one CTA, or of a cluster of them, for the whole
+ * chain). */
 int fft3d_b200_chain_run(fft3d_b200_chain *chain, const void *d_x0, void *d_out, long long steps,
                          void *stream);
+
+/* How the chain runs: CTAs a volume, and up to how many volumes have a cluster each. */
+const char *fft3d_b200_chain_describe(const fft3d_b200_chain *chain);
 
 void fft3d_b200_chain_destroy(fft3d_b200_chain *chain);
 
@@ -290,6 +294,10 @@ int fft3d_b200_server_drain(fft3d_b200_server *server, double timeout_s);
 
 /* Latency percentiles and throughput of everything finished so far. */
 int fft3d_b200_server_get_stats(fft3d_b200_server *server, fft3d_b200_server_stats *stats);
+
+/* Launches over lists of 36^3 volumes so far: where that is shorter than running them
+ * as items of the batch launch, a batch's cubes of a precision take one beside it. */
+long long fft3d_b200_server_list_launches(fft3d_b200_server *server);
 
 /* Per-request latencies of the first `max` finished requests, in completion
  * order: tickets[k] finished latency_s[k] seconds after its submission (host

@@ -10,9 +10,12 @@
 // fused into its epilogue, written back in place -- and writes the end state to
 // HBM once.  A whole chain is one launch; HBM traffic is one read of the start
 // state (plus the map constant, which stays in L2) and one write of the end.
+// A few 17^3 or 24^3 volumes, which would leave most SMs idle, run on a cluster of
+// four CTAs each (k_chain_cluster).
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstdio>
 #include <string>
 #include <vector>
 
@@ -236,6 +239,7 @@ struct fft3d_b200_chain {
     const void *cmap;
     const ChainEntry *e;
     bool cluster;
+    std::string describe;
     double uscale;
 };
 
@@ -259,7 +263,8 @@ extern "C" int fft3d_b200_chain_create(int n0, int n1, int n2, long long batch, 
     if (device < 0) device = prev < 0 ? 0 : prev;
     if (cudaSetDevice(device) != cudaSuccess) return FFT3D_B200_ERR_CUDA;
     int st = ensure_device_tables(device);
-    const bool cluster = st == FFT3D_B200_OK && e->cl > 0 && batch <= chain_clusters(*e);
+    const int most = st == FFT3D_B200_OK && e->cl > 0 ? chain_clusters(*e) : 0;
+    const bool cluster = batch <= most;
     if (st == FFT3D_B200_OK &&
         cudaFuncSetAttribute(e->func, cudaFuncAttributeMaxDynamicSharedMemorySize, e->smem) !=
             cudaSuccess) {
@@ -279,6 +284,16 @@ extern "C" int fft3d_b200_chain_create(int n0, int n1, int n2, long long batch, 
     c->cmap = d_c;
     c->e = e;
     c->cluster = cluster;
+    char buf[160];
+    int len = snprintf(buf, sizeof buf, "chain %dx%dx%d %s, ", n0, n1, n2,
+                       precision == FFT3D_B200_C128 ? "double" : "float");
+    if (cluster) snprintf(buf + len, sizeof buf - len, "a cluster of %d CTAs a volume", e->cl);
+    else snprintf(buf + len, sizeof buf - len, "one CTA a volume");
+    c->describe = buf;
+    if (most > 0) {
+        snprintf(buf, sizeof buf, " (up to %d volumes in clusters)", most);
+        c->describe += buf;
+    }
     c->uscale = 1.0 / std::sqrt((double)n0 * n1 * n2);
     *out = c;
     return FFT3D_B200_OK;
@@ -324,6 +339,11 @@ extern "C" int fft3d_b200_chain_run(fft3d_b200_chain *c, const void *d_x0, void 
         err = cudaLaunchKernelExC(&cfg, func, args);
     }
     return err == cudaSuccess ? FFT3D_B200_OK : FFT3D_B200_ERR_CUDA;
+}
+
+extern "C" const char *fft3d_b200_chain_describe(const fft3d_b200_chain *c)
+{
+    return c ? c->describe.c_str() : "";
 }
 
 extern "C" void fft3d_b200_chain_destroy(fft3d_b200_chain *c) { delete c; }

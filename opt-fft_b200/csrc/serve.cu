@@ -115,6 +115,7 @@ struct fft3d_b200_server {
     std::deque<unsigned long long> completed;
     unsigned long long next_ticket = 1;
     unsigned long long submitted = 0, finished = 0;
+    std::atomic<long long> list_launches{0};
     std::atomic<bool> stall_list{false};  // fft3d_b200_debug_stall_next_list
     std::atomic<bool> stop{false};
     std::thread thr;
@@ -195,6 +196,7 @@ static int launch_cubes(fft3d_b200_server *s, ServeSlot &slot, int precision, lo
         launch_entry(e, slot.d_items + first, nullptr, n, 1.0 / (36.0 * 36.0 * 36.0), slot.stream, grid,
                      slot.d_err, slot.d_scratch) != cudaSuccess)
         return FFT3D_B200_ERR_CUDA;
+    s->list_launches.fetch_add(1, std::memory_order_relaxed);
     return FFT3D_B200_OK;
 }
 
@@ -636,6 +638,11 @@ extern "C" int fft3d_b200_server_get_stats(fft3d_b200_server *s, fft3d_b200_serv
         out->span_s = span;
     }
     return s->status;
+}
+
+extern "C" long long fft3d_b200_server_list_launches(fft3d_b200_server *s)
+{
+    return s ? s->list_launches.load(std::memory_order_relaxed) : FFT3D_B200_ERR_INVALID;
 }
 
 extern "C" long long fft3d_b200_server_latencies(fft3d_b200_server *s, unsigned long long *tickets,

@@ -110,12 +110,12 @@ EXPORTS = {
                      "fft3d_b200_batch_describe", "fft3d_b200_batch_execute_noalloc",
                      "fft3d_b200_noalloc_check",
                      "fft3d_b200_chain_create", "fft3d_b200_chain_run",
-                     "fft3d_b200_chain_destroy",
+                     "fft3d_b200_chain_describe", "fft3d_b200_chain_destroy",
                      "fft3d_b200_server_create", "fft3d_b200_server_submit",
                      "fft3d_b200_server_submit_many",
                      "fft3d_b200_server_poll", "fft3d_b200_server_drain",
                      "fft3d_b200_server_get_stats", "fft3d_b200_server_latencies",
-                     "fft3d_b200_debug_stall_next_list", "fft3d_b200_server_destroy"],
+                     "fft3d_b200_server_list_launches", "fft3d_b200_debug_stall_next_list", "fft3d_b200_server_destroy"],
 }
 
 
@@ -191,6 +191,8 @@ def _load():
         "fft3d_b200_server_get_stats": ([vp, ctypes.POINTER(ServerStats)], i),
         "fft3d_b200_server_latencies": ([vp, ctypes.POINTER(ctypes.c_ulonglong),
                                          ctypes.POINTER(ctypes.c_double), ll], ll),
+        "fft3d_b200_chain_describe": ([vp], ctypes.c_char_p),
+        "fft3d_b200_server_list_launches": ([vp], ll),
         "fft3d_b200_debug_stall_next_list": ([vp], i),
         "fft3d_b200_server_destroy": ([vp], None),
     }
@@ -463,6 +465,9 @@ class Chain:
         _check(_lib.fft3d_b200_chain_run(self._h, d_x0, d_out, int(steps), stream or None),
                "chain_run")
 
+    def describe(self) -> str:
+        return _lib.fft3d_b200_chain_describe(self._h).decode()
+
     def close(self):
         if getattr(self, "_h", None):
             _lib.fft3d_b200_chain_destroy(self._h)
@@ -549,6 +554,10 @@ class Server:
         st = ServerStats()
         _check(_lib.fft3d_b200_server_get_stats(self._h, ctypes.byref(st)), "server_stats")
         return {name: getattr(st, name) for name, _ in ServerStats._fields_}
+
+    def list_launches(self) -> int:
+        """Launches over lists of 36^3 volumes so far."""
+        return _lib.fft3d_b200_server_list_launches(self._h)
 
     def close(self):
         if getattr(self, "_h", None):

@@ -26,6 +26,10 @@ def steps_of(x, c, m):
     return x
 
 
+def clusters_at_once(chain):
+    return int(chain.describe().split("up to ")[1].split()[0])
+
+
 @pytest.mark.parametrize("side,batch", [(17, 1), (17, 30), (17, 37), (24, 2), (24, 33), (24, 38)])
 @pytest.mark.parametrize("prec", [fb.C128, fb.C64])
 @pytest.mark.parametrize("kind", [fb.CHAIN_UNITARY, fb.CHAIN_MAP])
@@ -38,6 +42,9 @@ def test_chain(side, batch, prec, kind):
     dc = torch.from_numpy(c).cuda() if c is not None else None
     out = torch.empty_like(a)
     chain = fb.Chain((side,) * 3, batch, kind, prec, dc.data_ptr() if dc is not None else 0)
+    most = clusters_at_once(chain)
+    assert most >= 30  # of the B200's 37 groups of four SMs
+    assert ("a cluster of 4 CTAs a volume" in chain.describe()) == (batch <= most), chain.describe()
     pick = sorted({0, batch // 2, batch - 1})
     for m in (0, 1, 3):
         out.zero_()
@@ -47,3 +54,23 @@ def test_chain(side, batch, prec, kind):
         err = oracle.rel_error_per_volume(out.cpu().numpy()[pick].astype(np.complex128), want).max()
         assert err <= TOL[prec] * max(m, 1), (m, err)
     chain.close()
+
+
+@pytest.mark.parametrize("side,prec", [(17, fb.C128), (17, fb.C64), (24, fb.C128), (24, fb.C64)])
+def test_both_sides_of_the_line(side, prec):
+    """As many volumes as have a cluster each, and one more; the smaller cubes have none."""
+    dt = np.complex128 if prec == fb.C128 else np.complex64
+    chain = fb.Chain((side,) * 3, 1, fb.CHAIN_UNITARY, prec)
+    most = clusters_at_once(chain)
+    for batch, cluster in ((most, True), (most + 1, False)):
+        x = field(np.random.default_rng(batch), (batch, side, side, side), dtype=dt)
+        a = torch.from_numpy(x).cuda()
+        out = torch.zeros_like(a)
+        chain = fb.Chain((side,) * 3, batch, fb.CHAIN_UNITARY, prec)
+        assert ("cluster of 4" in chain.describe()) == cluster
+        chain.run(a.data_ptr(), out.data_ptr(), 2)
+        torch.cuda.synchronize()
+        err = oracle.rel_error_per_volume(out.cpu().numpy()[-2:].astype(np.complex128),
+                                          steps_of(x[-2:].astype(np.complex128), None, 2)).max()
+        assert err <= 2 * TOL[prec], err
+    assert "one CTA a volume" in fb.Chain((16, 16, 16), 1, fb.CHAIN_UNITARY, prec).describe()
