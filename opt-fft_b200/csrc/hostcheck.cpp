@@ -877,8 +877,6 @@ extern "C" int hostcheck_tpass(int tl, int sign, void *data, long long vol_elems
     return -2;
 }
 
-// Items whose dependency wait would not hold when taken in ticket order (the
-// TWOPASS deadlock-freedom argument); reset by reading.
 // LitTw<n> and the table's entries of length n, {cos, sin} each.
 extern "C" int hostcheck_literal_factors(int n, double *lit, double *tab)
 {
@@ -893,6 +891,8 @@ extern "C" int hostcheck_literal_factors(int n, double *lit, double *tab)
     return 0;
 }
 
+// Items whose dependency wait would not hold when taken in ticket order (the
+// TWOPASS deadlock-freedom argument); reset by reading.
 extern "C" long long hostcheck_twopass_violations()
 {
     const long long v = g_twopass_violations;

@@ -78,9 +78,9 @@ struct ServeSlot {
     unsigned int *d_ticket = nullptr;
     unsigned char *d_solo = nullptr;
     unsigned char *d_scratch = nullptr;
-    // The slot's error word, in mapped host memory: kernels write it only when a bounded
-    // wait runs out, and the host reads it when the slot's event has passed, without a
-    // copy in the stream of every launch.
+    // The slot's error word, one of the server's in mapped host memory: kernels write it
+    // only when a bounded wait runs out, and the host reads it when the slot's event has
+    // passed, without a copy in the stream of every launch.
     volatile int *h_err = nullptr;
     int *d_err = nullptr;          // its device address
     int status = FFT3D_B200_OK;    // of the launch calls
@@ -108,6 +108,7 @@ struct fft3d_b200_server {
     long long scratch_per_cta = 0;
     int cube_grid[2] = {0, 0};  // CTAs of a list launch, by precision
     std::vector<ServeSlot> slots;
+    int *h_errs = nullptr;  // the slots' error words
     std::mutex mu;
     std::condition_variable cv;
     std::deque<ServeReq> pending;
@@ -424,10 +425,10 @@ static void server_free(fft3d_b200_server *s)
         cudaFree(slot.d_ticket);
         cudaFree(slot.d_solo);
         cudaFree(slot.d_scratch);
-        if (slot.h_err) cudaFreeHost(const_cast<int *>(slot.h_err));
         if (slot.h_items) cudaFreeHost(slot.h_items);
         if (slot.h_segs) cudaFreeHost(slot.h_segs);
     }
+    if (s->h_errs) cudaFreeHost(s->h_errs);
     delete s;
 }
 
@@ -478,13 +479,18 @@ extern "C" int fft3d_b200_server_create(size_t hbm_budget_bytes, int max_infligh
         scratch_bytes = std::max(scratch_bytes, entry_workspace_bytes(e, s->cube_grid[k]));
     }
     s->slots.resize((size_t)max_inflight);
+    int *d_errs = nullptr;
+    if (cudaHostAlloc(&s->h_errs, sizeof(int) * (size_t)max_inflight, cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer(&d_errs, s->h_errs, 0) != cudaSuccess)
+        return fail(FFT3D_B200_ERR_NOMEM);
     for (ServeSlot &slot : s->slots) {
+        const size_t i = (size_t)(&slot - s->slots.data());
+        s->h_errs[i] = 0;
+        slot.h_err = s->h_errs + i;
+        slot.d_err = d_errs + i;
         if (cudaStreamCreateWithFlags(&slot.stream, cudaStreamNonBlocking) != cudaSuccess ||
-            cudaEventCreateWithFlags(&slot.done, cudaEventDisableTiming) != cudaSuccess ||
-            cudaHostAlloc((void **)&slot.h_err, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
-            cudaHostGetDevicePointer((void **)&slot.d_err, const_cast<int *>(slot.h_err), 0) != cudaSuccess)
+            cudaEventCreateWithFlags(&slot.done, cudaEventDisableTiming) != cudaSuccess)
             return fail(FFT3D_B200_ERR_NOMEM);
-        *slot.h_err = 0;
         if (!(flags & FFT3D_B200_SERVE_PLAIN)) {
             if (cudaMalloc(&slot.d_items, sizeof(BatchItem) * SERVE_MAX_ITEMS) != cudaSuccess ||
                 cudaMalloc(&slot.d_segs, sizeof(BatchSeg) * SERVE_MAX_SEGS) != cudaSuccess ||

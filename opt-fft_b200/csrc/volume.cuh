@@ -114,8 +114,8 @@ FFT_HD cx<T> load_in(const cx<T> *p)
 }
 
 // x lines of a prime length above 31 (47, 83 and 97 among the reference's test
-// extents; on the GPU they are LONG's, longline.cuh, and these passes are what
-// its results are compared with): a folded sum held in registers would spill kilobytes a thread, so
+// extents), one line a thread: run on the CPU by the tests only, since on the GPU
+// they are LONG's (longline.cuh).  A folded sum held in registers would spill kilobytes a thread, so
 // the line is summed straight out of shared memory, one output at a time, with
 // double twiddles and accumulators; only x-pass lines are that long.
 constexpr bool x_direct_sum(int n) { return ce_is_prime(n) && n > 31; }
