@@ -13,7 +13,8 @@
 // 33.5, 8x8x1 (as 1x8x8) c128 66.9 / 35.7 and c64 48.4 / 39.0.  Of some
 // 900 shapes swept (2-4 stages, 1-8 CTAs an SM, register or bulk stores) the
 // fastest of each extent is kept, and a second one with smaller items where that
-// costs under 7%, for batches that the larger items would leave on few SMs.  The
+// costs under 7%, for batches that the larger items would leave on few SMs.  (4^3
+// complex double and 8x1x8 complex float have VOLUME alone.)  The
 // VOLUME kernels stay in the tuner's race: at under a few hundred volumes their
 // one pass per CTA is up to 20% shorter (9x25x7 c128 x 20: 3.5 / 4.1 us).
 #include "stream.cuh"
