@@ -18,8 +18,8 @@ def rule(hostcheck):
 def estimate(way, n, other_bytes, sms):
     lists = sum(12 + us * k for bit, us, k in ((1, 0.48, n[0]), (2, 0.26, n[1])) if way & bit)
     a, b = (0 if way & bit else k for bit, k in ((1, n[0]), (2, n[1])))
-    # items of 98 and 49 us, largest first, on `sms` SMs
-    last = max(98 * math.ceil(a / sms), 49 * math.ceil((2 * a + b) / sms))
+    # items of 98 and 49 us on `sms` SMs, those with one of 98 taking part in the second round
+    last = 49 * (math.ceil(a / sms) + math.ceil((a + b) / sms))
     return lists + max(last, other_bytes / 2.3e6 + (98 * a + 49 * b) / sms)
 
 
@@ -36,8 +36,8 @@ def test_shortest_of_the_four(rule):
 
 @pytest.mark.parametrize("sms,n128,n64,other_mb,way", [
     (148, 0, 0, 0, 0), (148, 1, 0, 0, 1), (148, 0, 1, 0, 2), (148, 64, 64, 0, 3), (148, 2, 3, 500, 0),
-    # one precision's cubes are among the other's batch: each alone would take a list here
-    (148, 3, 161, 98, 0), (148, 1, 149, 180, 0),
+    # the precisions together: 7 alone would take a list, and so would 82; 13 and 145 are more than one round
+    (148, 7, 81, 157, 0), (148, 82, 7, 82, 0), (148, 13, 145, 94, 1), (148, 12, 191, 167, 0),
     # the device's own SMs: 30 volumes are two rounds of 20
     (148, 30, 0, 150, 1), (20, 30, 0, 150, 1), (148, 30, 0, 300, 0), (20, 30, 0, 300, 1)])
 def test_examples(rule, sms, n128, n64, other_mb, way):
